@@ -256,44 +256,56 @@ __device__ __forceinline__ CellGrid cell_grid(const Dev& d, int i)
 // value the previous step's limit reduction left in dtv
 __device__ __forceinline__ double step_dt(const Dev& d) { return d.p.cfl_on ? *d.s.dtv : d.p.dt; }
 
+// A 32-byte record moved by one 256-bit access (sm_100's widest).  The
+// records of consecutive particles are consecutive, so a warp's access is
+// whole lines; as two 16-byte loads each instruction touched every second 16
+// bytes of twice the lines, and the passes that gather most (stress
+// divergence, viscosity) sat at 82-87% of the L1 pipe.  The record arrays are
+// whole cudaMalloc allocations, so every record is 32-byte aligned.
+struct alignas(32) Rec4 { double a, b, c, e; };
+__device__ __forceinline__ Rec4 ld_rec4(const double* base, size_t rec)
+{
+    Rec4 r;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(r.a), "=d"(r.b), "=d"(r.c), "=d"(r.e) : "l"(base + 4 * rec));
+    return r;
+}
+__device__ __forceinline__ void st_rec4(double* base, size_t rec, double a, double b, double c, double e)
+{
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};"
+                 ::"l"(base + 4 * rec), "d"(a), "d"(b), "d"(c), "d"(e) : "memory");
+}
+
 __device__ __forceinline__ Pos load_pos(const double* xh, int i)
 {
-    const double2* p = reinterpret_cast<const double2*>(xh) + 2 * (size_t)i;
-    double2 a = p[0], b = p[1];
-    return Pos{a.x, a.y, b.x, b.y};
+    const Rec4 r = ld_rec4(xh, (size_t)i);
+    return Pos{r.a, r.b, r.c, r.e};
 }
 
 // the momentum record of particle j (DevState::sr)
 struct SR { double s[6], p, m; };
 __device__ __forceinline__ SR load_sr(const double* sr, int j)
 {
-    const double2* q = reinterpret_cast<const double2*>(sr) + 4 * (size_t)j;
-    const double2 a = q[0], b = q[1], c = q[2], e = q[3];
-    return SR{{a.x, a.y, b.x, b.y, c.x, c.y}, e.x, e.y};
+    const Rec4 a = ld_rec4(sr, 2 * (size_t)j), b = ld_rec4(sr, 2 * (size_t)j + 1);
+    return SR{{a.a, a.b, a.c, a.e, b.a, b.b}, b.c, b.e};
 }
 __device__ __forceinline__ void store_sr(double* sr, int i, const double s[6], double p, double m)
 {
-    double2* q = reinterpret_cast<double2*>(sr) + 4 * (size_t)i;
-    q[0] = make_double2(s[0], s[1]);
-    q[1] = make_double2(s[2], s[3]);
-    q[2] = make_double2(s[4], s[5]);
-    q[3] = make_double2(p, m);
+    st_rec4(sr, 2 * (size_t)i, s[0], s[1], s[2], s[3]);
+    st_rec4(sr, 2 * (size_t)i + 1, s[4], s[5], p, m);
 }
 
 // the neighbour record of particle j: vxp (x, y, z) and mass
 struct NV { double vx, vy, vz, m; };
 __device__ __forceinline__ NV load_nv(const double* nv, int j)
 {
-    const double2* p = reinterpret_cast<const double2*>(nv) + 2 * (size_t)j;
-    double2 a = p[0], b = p[1];
-    return NV{a.x, a.y, b.x, b.y};
+    const Rec4 r = ld_rec4(nv, (size_t)j);
+    return NV{r.a, r.b, r.c, r.e};
 }
 
 __device__ __forceinline__ void store_pos(double* xh, int i, const Pos& q)
 {
-    double2* p = reinterpret_cast<double2*>(xh) + 2 * (size_t)i;
-    p[0] = make_double2(q.x, q.y);
-    p[1] = make_double2(q.z, q.h);
+    st_rec4(xh, (size_t)i, q.x, q.y, q.z, q.h);
 }
 
 // the normalisation constant a1 of weight() / weight2() for support ra
@@ -469,9 +481,8 @@ __device__ __forceinline__ double wall_vel(const Dev& d, int ti, int j, const do
 // corrected in place by kernel_gradient_correction when flknl is 3 or 4.
 __device__ __forceinline__ void load_w_raw(const double* nbw, int N, int s, int i, double w[4])
 {
-    const double2* p = reinterpret_cast<const double2*>(nbw) + 2 * ((size_t)s * N + i);
-    const double2 a = p[0], b = p[1];
-    w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
+    const Rec4 r = ld_rec4(nbw, (size_t)s * N + i);
+    w[0] = r.a; w[1] = r.b; w[2] = r.c; w[3] = r.e;
 }
 __device__ __forceinline__ void load_w_raw(const double* nbw, int N, int s, int i, float w[4])
 {
@@ -494,9 +505,7 @@ __device__ __forceinline__ void pair_value(const Dev& d, const PairI<R>& I, R rr
 
 __device__ __forceinline__ void store_w(const Dev& d, int s, int i, const double w[4])
 {
-    double2* p = reinterpret_cast<double2*>(d.s.nbw) + 2 * ((size_t)s * d.p.N + i);
-    p[0] = make_double2(w[0], w[1]);
-    p[1] = make_double2(w[2], w[3]);
+    st_rec4(d.s.nbw, (size_t)s * d.p.N + i, w[0], w[1], w[2], w[3]);
 }
 __device__ __forceinline__ void store_w(const Dev& d, int s, int i, const float w[4])
 {

@@ -661,16 +661,12 @@ __global__ void __launch_bounds__(128, SPH_MINB_PAIRW) k_pairw(Dev d)
         // k_density's record of the porosity gathers: mass, porosity, rho of
         // the last step and its reciprocal (for the divisions by rho_j)
         const double r = d.s.rho[i];
-        double2* q = reinterpret_cast<double2*>(d.s.rrho) + 2 * (size_t)i;
-        q[0] = make_double2(d.s.mass[i], d.s.porosity[i]);
-        q[1] = make_double2(r, 1.0 / r);
+        st_rec4(d.s.rrho, (size_t)i, d.s.mass[i], d.s.porosity[i], r, 1.0 / r);
     }
     {
         // the neighbour record of this step (vxp and mass change only between steps)
         const int N = d.p.N;
-        double2* q = reinterpret_cast<double2*>(d.s.nv) + 2 * (size_t)i;
-        q[0] = make_double2(d.s.vxp[i], d.s.vxp[N + i]);
-        q[1] = make_double2(d.s.vxp[2 * N + i], d.s.mass[i]);
+        st_rec4(d.s.nv, (size_t)i, d.s.vxp[i], d.s.vxp[N + i], d.s.vxp[2 * N + i], d.s.mass[i]);
     }
     if (d.p.bulk) pairw_particle<ND, float>(d, i);
     else pairw_particle<ND, double>(d, i);
@@ -808,9 +804,7 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_shepard_eos(Dev d)
     d.s.rho[i] = r;
     {
         // the strain loop's neighbour record: vxp and mass / rho of this step
-        double2* q = reinterpret_cast<double2*>(d.s.svr) + 2 * (size_t)i;
-        q[0] = make_double2(d.s.vxp[i], d.s.vxp[N + i]);
-        q[1] = make_double2(d.s.vxp[2 * N + i], d.s.mass[i] / r);
+        st_rec4(d.s.svr, (size_t)i, d.s.vxp[i], d.s.vxp[N + i], d.s.vxp[2 * N + i], d.s.mass[i] / r);
     }
     const double prep = d.s.prep[i];
     if (ti == 1) {
@@ -826,9 +820,7 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_shepard_eos(Dev d)
     }
     {
         // the pressure gathers' record: mass, rho and pressure of this step
-        double2* q = reinterpret_cast<double2*>(d.s.pmr) + 2 * (size_t)i;
-        q[0] = make_double2(d.s.mass[i], r);
-        q[1] = make_double2(d.s.pre[i], 0.0);
+        st_rec4(d.s.pmr, (size_t)i, d.s.mass[i], r, d.s.pre[i], 0.0);
     }
 }
 
@@ -1269,9 +1261,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRESS) k_stress(Dev d)
     {
         // the drag loop's record: rho, saturation, porosity, and the soil's
         // permeability or the fluid's density
-        double2* q = reinterpret_cast<double2*>(d.s.dr4) + 2 * (size_t)i;
-        q[0] = make_double2(r, d.s.satu[i]);
-        q[1] = make_double2(d.s.porosity[i], (ti == 2) ? d.s.cop[i] : d.s.f_dens[i]);
+        st_rec4(d.s.dr4, (size_t)i, r, d.s.satu[i], d.s.porosity[i], (ti == 2) ? d.s.cop[i] : d.s.f_dens[i]);
     }
 }
 
@@ -2008,9 +1998,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_ACCB) k_accel_b_tail(Dev d)
     }
     for (int k = 0; k < 3; k++) d.s.ax[k * N + i] = ax[k];
     // the velocity before XSPH, with the mass, as one record for XSPH's gathers
-    double2* vq = reinterpret_cast<double2*>(d.s.vx_next) + 2 * (size_t)i;
-    vq[0] = make_double2(vout[0], vout[1]);
-    vq[1] = make_double2(vout[2], d.s.mass[i]);
+    st_rec4(d.s.vx_next, (size_t)i, vout[0], vout[1], vout[2], d.s.mass[i]);
 }
 
 // xsph (CPP_11-xsph.cpp:145-256, Jacobi by construction: reads the velocities
