@@ -276,6 +276,7 @@ void fill_dev_params(DevParams& p, const sphgpu_params* P)
     p.cfl_on = 0; p.cfl_c = 0.0; p.cfl_f = 0.0;
     p.st_vpu = P->structure.vpu;
     p.ninst = 0;
+    p.split = p.ss_coupled ? 0 : 1;
     for (int q = 0; q < TP_COUNT; q++) p.tb[q] = 128;
     p.flr = P->flr == 1 ? 1 : 0;
     p.rain_lp = 0; p.rain_vrain = 0.0; p.rain_press = 0.0;
@@ -956,7 +957,7 @@ sphgpu_ctx* sphgpu_create(const sphgpu_params* P, int device)
     r |= dalloc(c, &s.nps, N); r |= dalloc(c, &s.sortpos, N); r |= dalloc(c, &s.pts, N);
     if (!s.accb) r |= dalloc(c, &s.accb, 9 * (size_t)N);   // (19N when alloc_optional sized it for vibration)
     r |= dalloc(c, &s.nbrs, (size_t)SPH_NB_CAP * N);
-    r |= dalloc(c, &s.nbm, 10 * (size_t)N);
+    r |= dalloc(c, &s.nab, N); r |= dalloc(c, &s.nbm, 2 * (size_t)N);
     r |= dalloc(c, &s.nbw, 4 * (size_t)SPH_NB_CAP * N);
     r |= dalloc(c, &s.err, 1); r |= dalloc(c, &s.step, 1);
     r |= dalloc(c, &s.dtv, 1); r |= dalloc(c, &s.dtmin, 1); r |= dalloc(c, &s.nrain, 1); r |= dalloc(c, &s.tsim, 1);
@@ -2272,7 +2273,10 @@ int sphgpu_nnps(sphgpu_ctx* c, int* ninflu, int* influ)
     if (c->sticky) return c->sticky;
     cudaSetDevice(c->device);
     if (const int ro = to_caller_order(c)) return ro;
-    sphk_enqueue_nnps(&c->d[c->parity], c->sort_tmp, c->sort_bytes, c->end_bit, c->st, nullptr);
+    // the lists whole, in list order
+    Dev whole = c->d[c->parity];
+    whole.p.split = 0;
+    sphk_enqueue_nnps_parts(&whole, c->sort_tmp, c->sort_bytes, c->end_bit, c->st, nullptr, 3);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->st));
     int err = 0;
@@ -2287,8 +2291,14 @@ int sphgpu_nnps(sphgpu_ctx* c, int* ninflu, int* influ)
             int* row = influ + (size_t)i * 100;
             std::memset(row, 0, sizeof(int) * 100);
             const int m = cnt[i] < SPH_NB_CAP ? cnt[i] : SPH_NB_CAP;
-            for (int s = 0; s < m; s++) row[s + 1] = nb[(size_t)s * N + i];
+            for (int s = 0; s < m; s++) row[s + 1] = nb[(size_t)s * N + i] >> 3;
         }
+    }
+    if (c->part_done >= 2 && err == 0) {
+        // the lists of the step that sphgpu_update will complete
+        sphk_enqueue_nnps_parts(&c->d[c->parity], c->sort_tmp, c->sort_bytes, c->end_bit, c->st, nullptr, 2);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(c->st));
     }
     return err;
 }

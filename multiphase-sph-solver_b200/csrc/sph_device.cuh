@@ -9,11 +9,19 @@
 //   * vectors:   double a[3 * N], component k of particle i at a[k * N + i]
 //   * tensors:   double a[6 * N] (Voigt order xx yy zz xy yz zx, as
 //                Particle::sig), component k at a[k * N + i]
-//   * neighbour lists: int nbr[SPH_NB_CAP * N], slot s of particle i at
-//                nbr[s * N + i], so the threads of a warp read consecutive
-//                words per slot; the pair's kernel gradient and value
-//                (Par_Cell::wij) in the same slot order, nbw[s * N + i], as a
-//                32-byte FP64 record or a 16-byte FP32 record (bulk form).
+//   * neighbour lists: int nbr[SPH_NB_CAP * N], row r of particle i at
+//                nbr[r * N + i], so the threads of a warp read consecutive
+//                words per row; a word is the neighbour's index << 3 | its
+//                type code.  A particle's list is held in two groups, each in
+//                the reference's list order: group A in rows 0, 1, ... (the
+//                types its gradient sums run over: for a solid the walls and
+//                the solids, for a fluid the walls and the fluids, for a wall
+//                the walls), group B in rows 98, 97, ... (the other types,
+//                whose sums need only the kernel value)
+//   * pair records (Par_Cell::wij): planes of SPH_NB_CAP * N values in the
+//                list's rows, nbw[(k * SPH_NB_CAP + r) * N + i], k = 0..2 the
+//                kernel gradient (group A only), 3 the kernel value; FP64, or
+//                FP32 in the bulk form.
 // Component-major storage makes every own-particle load of one component a
 // coalesced 8-byte-per-lane access.
 //
@@ -88,6 +96,8 @@ struct DevParams {
     double cfl_c, cfl_f;       // factors of h / (c + |v|) and sqrt(h / |a|)
     double st_vpu;             // Para_Structure::vpu, the structure's sound speed
     int ninst;                 // batched context: number of instances (0: one system)
+    int split;                 // 1: the lists in their two groups; 0: all of a list in group A, in list
+                               // order (coupled_Water_Soil_Structure's sums run over both groups' types)
     int tb[TP_COUNT];          // threads per block of the tuned passes
     // rainfall (flr 1, rtype 1): rainini's lp and vrain, Para_Rain::press_factor
     int flr, rain_lp;
@@ -208,14 +218,10 @@ struct DevState {
     // update (StiffMat::depp0, CPP_7-2-constitutive.cpp:112-292), N; and
     // Para_Vibra::loads, vib_nsteps x 3
     double *stiff, *vib_loads;
-    // per particle and particle type t = 0..4, bit s set when list slot s
-    // holds a particle of type t: nbm[(2 t + w) * N + i], word w = 0 for
-    // slots 0-63, 1 for slots 64-98 (written by the search with the list)
-    unsigned long long* nbm;
-    int *nbr;                  // [SPH_NB_CAP * N]
-    double *nbw;               // pair records (grad W, W) of the neighbour-list slots, [SPH_NB_CAP * N]
-                               // records of 32 bytes (FP64), or 16 bytes (FP32, bulk form) in the
-                               // first half of the same buffer
+    int *nab;                  // per particle the rows of its groups: nA | nB << 8
+    unsigned long long* nbm;   // the rows of group A that hold walls: bit r of word r / 64, nbm[w * N + i]
+    int *nbr;                  // [SPH_NB_CAP * N], see the head of this file
+    double *nbw;               // pair record planes, see the head of this file
     // control words
     int *err;                  // first error code raised (0 = none)
     int *step;                 // Para_Pro::l of the step being run
@@ -463,6 +469,75 @@ __device__ __forceinline__ void pair_w_raw(const Dev& d, const PairI<R>& I, R rr
     }
 }
 
+// x / y as div_rcp gives it for finite operands, without branches; `bad`
+// collects whether a residual was not finite (the quotient is then the IEEE
+// division's business).  The tests are integer instructions, so that the FP64
+// pipe takes a multiply and two fused multiply-adds.
+__device__ __forceinline__ double div_rcp_fast(double x, double y, double yr, bool& bad)
+{
+    const double q = __dmul_rn(x, yr);
+    const double r = __fma_rn(-q, y, x);
+    const double v = __fma_rn(r, yr, q);
+    const int h = __double2hiint(r), l = __double2loint(r);
+    bad |= (h & 0x7ff00000) == 0x7ff00000;
+    return (((h << 1) | l) == 0) ? q : v;      // r = 0: q is exact, sign included
+}
+
+// pair_w_raw in FP64 for h_j = h_i, the same operations in the same order with
+// selects in place of the branches on s (a warp's pairs lie on both sides of
+// s = 1, so both sides ran anyway) and one test for all quotients in place of
+// one branch each: the pairs of several rows can then be interleaved (with two
+// rows at a time k_pairw takes 2.21 ms per step for 4.45 M particles, 3.19 with
+// pair_w_raw one row at a time).  GRAD: the gradient too.  Operands that take the IEEE division, and h_j != h_i, go
+// to pair_w_raw.
+template <int ND, bool GRAD>
+__device__ __forceinline__ void pair_w64(const Dev& d, const PairI<double>& I, double rra, const Pos& pj, double w[4])
+{
+    const double xj[3] = {pj.x, pj.y, pj.z};
+    double dx[3], dst = 0.0;
+#pragma unroll
+    for (int k = 0; k < ND; k++) {
+        dx[k] = I.x[k] - xj[k];
+        dst = dst + dx[k] * dx[k];
+    }
+    dst = sqrt(dst);
+    const double ra = I.h, a1 = I.a1;
+    bool bad = pj.h != ra;
+    const double s = div_rcp_fast(dst, ra, rra, bad);
+    const double D = ra * dst;
+    const double rD = GRAD ? __drcp_rn(D) : 0.0;
+    const double u = 2.0 - s;
+    const bool in = s <= 1.0, out = s > 1.0 && s <= 2.0, grad = s > 0.0;
+    const bool cubic = d.p.flknl == 1 || d.p.flknl == 3;
+    double vi, vo;
+    if (cubic) {
+        vi = a1 * (0.66666667 - s * s + 0.5 * s * s * s);
+        constexpr double r6 = 1.0 / 6.0;
+        vo = div_rcp_fast(a1 * u * u * u, 6.0, r6, bad);
+    } else {
+        vi = a1 * (6.0 - 6.0 * s + 1.0 * s * s * s);
+        vo = a1 * u * u * u;
+    }
+    // s < 0 cannot be; a NaN s fails both tests, as it fails pair_w_raw's
+    w[3] = in ? vi : out ? vo : 0.0;
+    if (GRAD) {
+        const double c = in ? a1 : a1 * (cubic ? -0.5 : -3.0);
+        const double p = cubic ? -2.0 * s + 1.5 * s * s : -6.0 + 3.0 * s * s;
+        const double m = in ? p : u;
+        w[2] = 0.0;
+        bool gbad = false;
+#pragma unroll
+        for (int k = 0; k < ND; k++) {
+            double t = c * dx[k] * m;
+            t = in ? t : t * u;
+            t = div_rcp_fast(t, D, rD, gbad);
+            w[k] = (grad && (in || out)) ? t : 0.0;
+        }
+        bad |= gbad && grad && (in || out);
+    }
+    if (bad) pair_w_raw<ND, double>(d, I, rra, pj, w);
+}
+
 // The virtual velocity component k of wall particle j seen by particle i of
 // type ti (CPP_6-density.cpp:89-121, CPP_7-1-strain.cpp:92-124): i's own
 // velocity with flbndy 1, the wall's per-phase velocity of tm_boundary with
@@ -476,40 +551,58 @@ __device__ __forceinline__ double wall_vel(const Dev& d, int ti, int j, const do
     return 0.0;
 }
 
-// The stored pair record of slot s of particle i: kernel gradient w[0..2] and
-// value w[3], as partisearching stores Par_Cell::wij (CPP_3-NNPS.cpp:339-345),
-// corrected in place by kernel_gradient_correction when flknl is 3 or 4.
-__device__ __forceinline__ void load_w_raw(const double* nbw, int N, int s, int i, double w[4])
-{
-    const Rec4 r = ld_rec4(nbw, (size_t)s * N + i);
-    w[0] = r.a; w[1] = r.b; w[2] = r.c; w[3] = r.e;
-}
-__device__ __forceinline__ void load_w_raw(const double* nbw, int N, int s, int i, float w[4])
-{
-    const float4 f = reinterpret_cast<const float4*>(nbw)[(size_t)s * N + i];
-    w[0] = f.x; w[1] = f.y; w[2] = f.z; w[3] = f.w;
-}
-__device__ __forceinline__ void load_w(const Dev& d, int s, int i, double w[4]) { load_w_raw(d.s.nbw, d.p.N, s, i, w); }
-__device__ __forceinline__ void load_w(const Dev& d, int s, int i, float w[4]) { load_w_raw(d.s.nbw, d.p.N, s, i, w); }
-// Slot s's pair record for a pass that needs only the kernel value w[3]:
-// with no kernel gradient correction (flknl 1, 2) recomputed from the
-// neighbour's position exactly as k_pairw computed it (the same operations on
-// the same values, so the same bits; the gradient's arithmetic, unused, is
-// dropped by the compiler), else the corrected record k_kgc left in nbw.
+// The stored pair record of list row r of particle i (off = r * N + i): kernel
+// gradient and value, as partisearching stores Par_Cell::wij
+// (CPP_3-NNPS.cpp:339-345), the gradient corrected in place by
+// kernel_gradient_correction when flknl is 3 or 4.  Each component is a plane
+// of its own: a warp reads 256 consecutive bytes per component, a pass that
+// needs only the value reads a quarter of the record, and 2-D runs read no
+// third component (it is zero).  Measured on B200, soil column of 4.45 M
+// particles, against 32-byte records in one list walked by type masks (ms per
+// step): strain 2.63 -> 1.75, XSPH 1.87 -> 1.18, Shepard 1.22 -> 0.66, density
+// 2.21 -> 1.48, stress divergence 2.13 -> 1.67, momentum loops 4.79 -> 4.15; the
+// passes were bound by the L1 pipe and by lanes of a warp on different rows.
 template <int ND, typename R>
-__device__ __forceinline__ void pair_value(const Dev& d, const PairI<R>& I, R rra, int j, int s, int i, R w[4])
+__device__ __forceinline__ void load_g(const Dev& d, size_t off, R w[3])
 {
-    if (d.p.flknl <= 2) pair_w_raw<ND, R>(d, I, rra, load_pos(d.s.xh, j), w);
-    else load_w(d, s, i, w);
+    const R* p = reinterpret_cast<const R*>(d.s.nbw) + off;
+    const size_t plane = (size_t)SPH_NB_CAP * d.p.N;
+    w[0] = p[0];
+    w[1] = p[plane];
+    w[2] = (ND == 3) ? p[2 * plane] : R(0);
 }
-
-__device__ __forceinline__ void store_w(const Dev& d, int s, int i, const double w[4])
+template <typename R>
+__device__ __forceinline__ R load_v(const Dev& d, size_t off)
 {
-    st_rec4(d.s.nbw, (size_t)s * d.p.N + i, w[0], w[1], w[2], w[3]);
+    return reinterpret_cast<const R*>(d.s.nbw)[3 * (size_t)SPH_NB_CAP * d.p.N + off];
 }
-__device__ __forceinline__ void store_w(const Dev& d, int s, int i, const float w[4])
+// The kernel value alone.  The bulk form's Shepard and porosity sums take it
+// recomputed from the neighbour's position with multiply-adds contracted (no
+// kernel gradient correction), as that form always has; the FP64 form reads
+// the record, which holds the same bits.
+template <int ND, typename R>
+__device__ __forceinline__ R pair_value(const Dev& d, const PairI<R>& I, R rra, int j, size_t off)
 {
-    reinterpret_cast<float4*>(d.s.nbw)[(size_t)s * d.p.N + i] = make_float4(w[0], w[1], w[2], w[3]);
+    if (sizeof(R) == 4 && d.p.flknl <= 2) {
+        R w[4];
+        pair_w_raw<ND, R>(d, I, rra, load_pos(d.s.xh, j), w);
+        return w[3];
+    }
+    return load_v<R>(d, off);
+}
+template <int ND, typename R>
+__device__ __forceinline__ void store_g(const Dev& d, size_t off, const R w[3])
+{
+    R* p = reinterpret_cast<R*>(d.s.nbw) + off;
+    const size_t plane = (size_t)SPH_NB_CAP * d.p.N;
+    p[0] = w[0];
+    p[plane] = w[1];
+    if (ND == 3) p[2 * plane] = w[2];
+}
+template <typename R>
+__device__ __forceinline__ void store_v(const Dev& d, size_t off, R v)
+{
+    reinterpret_cast<R*>(d.s.nbw)[3 * (size_t)SPH_NB_CAP * d.p.N + off] = v;
 }
 
 // x^7 rounded to nearest from a double-double product chain (Dekker's exact

@@ -131,89 +131,67 @@ __device__ __forceinline__ int cell_link(const CellGrid& g, int c, int slot)
     return (v <= 0 || v > g.ctotal) ? 0 : v + g.base;
 }
 
-__device__ __forceinline__ int nbr_count(const Dev& d, int i)
-{
-    int c = d.s.nnb[i];
-    return c > SPH_NB_CAP ? SPH_NB_CAP : c;
-}
-
-// The slot mask of particles of type t in particle i's list (word 0: slots
-// 0-63, word 1: slots 64-98); types 0-4 only (type 7 has none)
-struct SlotMask {
-    unsigned long long lo, hi;
-    __device__ __forceinline__ SlotMask operator|(const SlotMask& o) const { return SlotMask{lo | o.lo, hi | o.hi}; }
-    __device__ __forceinline__ bool any() const { return (lo | hi) != 0ull; }
-    __device__ __forceinline__ bool has(int s) const { return ((s < 64 ? lo >> s : hi >> (s - 64)) & 1ull) != 0; }
-};
-__device__ __forceinline__ SlotMask type_mask(const Dev& d, int i, int t)
-{
-    if (t < 0 || t > 4) return SlotMask{0ull, 0ull};
-    const size_t N = (size_t)d.p.N;
-    return SlotMask{d.s.nbm[(2 * t) * N + i], d.s.nbm[(2 * t + 1) * N + i]};
-}
-
-// The slots of particle i's list whose bits are set in a mask (from nbm:
-// one type's slots or a union), in slot order, with the next slot's particle index
-// loaded one slot ahead.  Lanes of a warp then take their k-th slot of the
-// class together, whatever the slots of other classes between them, so the
-// pass body runs with its lanes in step instead of idling on other classes.
-struct MaskIter {
-    const int* nbr;
-    size_t N;
-    int i, jn, sn;
-    unsigned long long m0, m1;
-    __device__ __forceinline__ int pop()
+// The rows of one group of particle i's list, in list order, the next row's
+// word loaded one row ahead.  A pass that sums over some of a group's types
+// skips the rows of the others; away from walls a group has one type, so the
+// lanes of a warp run row by row together on consecutive words and records.
+struct RowIter {
+    const int* p;              // the word after the prefetched one's
+    ptrdiff_t step;            // words from one row to the next: N, or -N in group B
+    size_t off;                // r * N + i of the prefetched row
+    int left, w1;
+    __device__ __forceinline__ RowIter(const Dev& d, int i, int n, int row0, int dir)
+        : step(dir * (ptrdiff_t)d.p.N), off((size_t)row0 * d.p.N + i), left(n)
     {
-        if (m0) { const int s = __ffsll(m0) - 1; m0 &= m0 - 1; return s; }
-        if (m1) { const int s = 63 + __ffsll(m1); m1 &= m1 - 1; return s; }
-        return -1;
+        p = d.s.nbr + off;
+        w1 = (n > 0) ? *p : 0;
     }
-    __device__ __forceinline__ MaskIter(const Dev& d, int i_, SlotMask m)
-        : nbr(d.s.nbr), N((size_t)d.p.N), i(i_), m0(m.lo), m1(m.hi)
+    // the next row's particle, type code and offset; false past the last
+    __device__ __forceinline__ bool next(int& j, int& tj, size_t& o)
     {
-        sn = pop();
-        jn = (sn >= 0) ? nbr[(size_t)sn * N + i] : 0;
-    }
-    // the next slot s and its particle j; false when the mask is exhausted
-    __device__ __forceinline__ bool next(int& s, int& j)
-    {
-        if (sn < 0) return false;
-        s = sn;
-        j = jn;
-        sn = pop();
-        if (sn >= 0) jn = nbr[(size_t)sn * N + i];
+        if (left <= 0) return false;
+        left--;
+        j = w1 >> 3;
+        tj = w1 & 7;
+        o = off;
+        off += step;
+        p += step;
+        if (left > 0) w1 = *p;
         return true;
     }
 };
+__device__ __forceinline__ RowIter rows_a(const Dev& d, int i) { return RowIter(d, i, d.s.nab[i] & 0xff, 0, 1); }
+// group B, or the whole list where it is not split
+__device__ __forceinline__ RowIter rows_b(const Dev& d, int i)
+{
+    const int n = d.s.nab[i];
+    return d.p.split ? RowIter(d, i, n >> 8, SPH_NB_CAP - 1, -1) : RowIter(d, i, n & 0xff, 0, 1);
+}
 
-// The list slots of particle i in order, each slot's particle index loaded
-// two slots ahead and its type one slot ahead.  A neighbour pass is a chain of
-// dependent loads per slot (list -> type -> the neighbour's fields); issuing
-// the first two for later slots while the current slot's gathers are in
-// flight leaves one load latency per slot instead of three.
-struct NbrIter {
-    const int* nbr;
-    const int* type;
-    size_t N;
-    int i, nn, s, j1, j2, t1;
-    __device__ __forceinline__ NbrIter(const Dev& d, int i_, int nn_)
-        : nbr(d.s.nbr), type(d.s.type), N((size_t)d.p.N), i(i_), nn(nn_), s(0)
+// the rows of group A that hold walls
+struct WallRows {
+    unsigned long long lo, hi;
+    __device__ __forceinline__ bool any() const { return (lo | hi) != 0ull; }
+    __device__ __forceinline__ int pop()
     {
-        j1 = (nn > 0) ? nbr[i] : 0;
-        j2 = (nn > 1) ? nbr[N + i] : 0;
-        t1 = (nn > 0) ? type[j1] : 0;
-    }
-    // slot s's particle and type; issues the loads of the slots after it
-    __device__ __forceinline__ void next(int& j, int& tj)
-    {
-        j = j1;
-        tj = t1;
-        j1 = j2;
-        t1 = (s + 1 < nn) ? type[j1] : 0;
-        j2 = (s + 2 < nn) ? nbr[(size_t)(s + 2) * N + i] : 0;
-        s++;
+        if (lo) { const int r = __ffsll(lo) - 1; lo &= lo - 1; return r; }
+        if (hi) { const int r = 63 + __ffsll(hi); hi &= hi - 1; return r; }
+        return -1;
     }
 };
+__device__ __forceinline__ WallRows wall_rows(const Dev& d, int i)
+{
+    return WallRows{d.s.nbm[i], d.s.nbm[(size_t)d.p.N + i]};
+}
+
+// the type codes (bits) that go to group A and group B of a particle of type t
+struct Groups { unsigned a, b; };
+__device__ __forceinline__ Groups list_groups(const Dev& d, int t)
+{
+    if (!d.p.split) return Groups{0xffu, 0u};
+    const unsigned a = (t == 0) ? 0x01u : (t == 1 || t == 3) ? 0x0bu : (t == 2 || t == 4) ? 0x15u : 0u;
+    return Groups{a, a ? 0x1fu & ~a : 0u};
+}
 
 // ---------------------------------------------------------------------------
 #ifndef SPH_BULK32
@@ -378,36 +356,6 @@ __global__ void k_cellrange(Dev d)
 // candidate to the FP64 path.  Only candidates within M of T^2 take the FP64
 // path, where the sqrt is evaluated only within 1e-10 of the squared radius,
 // so the decisions are those of the reference.
-// The per-type slot masks of one particle's list (nbm), built as the list
-// is written: bit s of word (t, s / 64) set when slot s holds type t (0-4)
-struct TypeMasks {
-    unsigned long long m[5][2];
-    __device__ __forceinline__ TypeMasks()
-    {
-#pragma unroll
-        for (int t = 0; t < 5; t++) m[t][0] = m[t][1] = 0ull;
-    }
-    __device__ __forceinline__ void add(int t, int s)
-    {
-        const unsigned long long lo = (s < 64) ? (1ull << s) : 0ull, hi = (s < 64) ? 0ull : (1ull << (s - 64));
-#pragma unroll
-        for (int k = 0; k < 5; k++)
-            if (t == k) {
-                m[k][0] |= lo;
-                m[k][1] |= hi;
-            }
-    }
-    __device__ __forceinline__ void store(const Dev& d, int i) const
-    {
-        const size_t N = (size_t)d.p.N;
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-            d.s.nbm[(2 * k) * N + i] = m[k][0];
-            d.s.nbm[(2 * k + 1) * N + i] = m[k][1];
-        }
-    }
-};
-
 // The FP64 inclusion test of one candidate, as partisearching decides it:
 // sqrt of the FP64 sum of squares against h_i + h_j, the sqrt evaluated only
 // within 1e-10 of the squared radius (outside that band the comparison of the
@@ -479,18 +427,51 @@ __device__ __forceinline__ int nnps_prefilter(const Prefilter& P, float4 fj)
     return -1;
 }
 
+// One particle's list as it is built: the rows of its two groups and the wall
+// rows of group A, in list order
+struct ListOut {
+    Groups g;
+    int cnt, na, nb;               // neighbours (of every type), rows of A and B
+    unsigned long long lo, hi;
+    __device__ __forceinline__ ListOut(const Dev& d, int t) : g(list_groups(d, t)), cnt(0), na(0), nb(0), lo(0ull), hi(0ull) {}
+    // word w = index << 3 | type code; past the capacity it is only counted
+    __device__ __forceinline__ void add(const Dev& d, int i, int w)
+    {
+        const int t = w & 7;
+        cnt++;
+        if (cnt > SPH_NB_CAP) return;
+        if ((g.a >> t) & 1u) {
+            if (t == 0) {
+                if (na < 64) lo |= 1ull << na;
+                else hi |= 1ull << (na - 64);
+            }
+            d.s.nbr[(size_t)na * d.p.N + i] = w;
+            na++;
+        } else if ((g.b >> t) & 1u) {
+            d.s.nbr[(size_t)(SPH_NB_CAP - 1 - nb) * d.p.N + i] = w;
+            nb++;
+        }
+    }
+    __device__ __forceinline__ void store(const Dev& d, int i) const
+    {
+        d.s.nnb[i] = cnt;
+        d.s.nab[i] = na | (nb << 8);
+        d.s.nbm[i] = lo;
+        d.s.nbm[(size_t)d.p.N + i] = hi;
+    }
+};
+
 // partisearching with every candidate decided in FP64 as soon as it is met
 // (used when the FP32 prefilter does not apply to the particle, or when its
-// provisional list below overflows); returns the neighbour count
+// provisional list below overflows)
 template <int ND>
-__device__ __forceinline__ int nnps_direct(const Dev& d, int i, int nc, const Pos& pi, bool fast, const Prefilter& P)
+__device__ __forceinline__ void nnps_direct(const Dev& d, int i, int nc, const Pos& pi, bool fast, const Prefilter& P,
+                                            ListOut& out)
 {
-    const int N = d.p.N;
     constexpr int nst = (ND == 2) ? 9 : 27;
     const double xi[3] = {pi.x, pi.y, pi.z};
     const float4* xsf = reinterpret_cast<const float4*>(d.s.xsf);
     const CellGrid g = cell_grid(d, i);
-    int cnt = 0;
     for (int nj = 0; nj < nst; nj++) {
         const int nl = cell_link<ND>(g, nc, nj);
         if (nl <= 0) continue;
@@ -499,16 +480,14 @@ __device__ __forceinline__ int nnps_direct(const Dev& d, int i, int nc, const Po
             int v = fast ? nnps_prefilter<ND>(P, xsf[q]) : -1;
             if (v < 0) v = nnps_in_fp64<ND>(xi, pi.h, load_pos(d.s.xs, q)) ? 1 : 0;
             if (v) {
-                const int j = d.s.pid_sorted[q];
-                if (i != j) {
-                    cnt++;
-                    if (cnt <= SPH_NB_CAP) d.s.nbr[(size_t)(cnt - 1) * N + i] = j;
-                    else raise_err(d.s.err, SPH_ERR_NEIGH);
+                const int w = d.s.pts[q];
+                if (i != (w >> 3)) {
+                    out.add(d, i, w);
+                    if (out.cnt > SPH_NB_CAP) raise_err(d.s.err, SPH_ERR_NEIGH);
                 }
             }
         }
     }
-    return cnt;
 }
 
 // partisearching (CPP_3-NNPS.cpp:265-374): neighbours of i in stencil order,
@@ -535,9 +514,8 @@ __device__ __forceinline__ int nnps_direct(const Dev& d, int i, int nc, const Po
 // list of its own sorted position, nbrs[s * N + q], which the lanes of a warp
 // fill row by row.  The resolve pass (k_nnps_resolve) runs one thread per
 // particle in the caller's order: it reads its provisional list, decides the
-// undecided candidates in FP64, and writes the list nbr[s * N + i] and the
-// per-type slot masks.  The order, and so the
-// list, is the one a single pass in candidate order gives.  A provisional list
+// undecided candidates in FP64, and writes the list into its two groups.  The
+// order within a group is the one a single pass in candidate order gives.  A provisional list
 // longer than the capacity (possible only when undecided candidates or the
 // particle itself push it over), and a particle the FP32 test does not apply
 // to, are searched again by the direct form, which also raises the
@@ -583,16 +561,15 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_nnps(Dev d)
     d.s.nps[q] = np;
 }
 
-// The resolve pass of the search (see k_nnps), one thread per particle, with
-// the per-type slot masks of the list written beside it.
+// The resolve pass of the search (see k_nnps), one thread per particle.
 template <int ND>
 __global__ void __launch_bounds__(128, SPH_MINB) k_nnps_resolve(Dev d)
 {
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
-    int cnt = 0;
-    TypeMasks tm;
-    if (d.s.type[i] != 7) {
+    const int ti = d.s.type[i];
+    ListOut out(d, ti);
+    if (ti != 7) {
         const int q0 = d.s.sortpos[i];
         const int np = d.s.nps[q0];
         const Pos pi = load_pos(d.s.xh, i);
@@ -603,9 +580,7 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_nnps_resolve(Dev d)
             float Fi = fmaxf(fabsf(fi.x), fabsf(fi.y));
             if (ND == 3) Fi = fmaxf(Fi, fabsf(fz));
             const Prefilter P = make_prefilter<ND>(fi.x, fi.y, fz, fi.w, 2.2f * U * Fi, 32.f * U);
-            cnt = nnps_direct<ND>(d, i, d.s.cell[i], pi, np >= 0, P);
-            const int nn = cnt < SPH_NB_CAP ? cnt : SPH_NB_CAP;
-            for (int s = 0; s < nn; s++) tm.add(d.s.type[d.s.nbr[(size_t)s * N + i]], s);
+            nnps_direct<ND>(d, i, d.s.cell[i], pi, np >= 0, P, out);
         } else {
             const double xi[3] = {pi.x, pi.y, pi.z};
             const int* row = d.s.nbrs + q0;
@@ -617,39 +592,72 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_nnps_resolve(Dev d)
                 if (s + 2 < np) v2 = row[(size_t)(s + 2) * N];
                 const int w = (v < 0) ? ~v : v, j = w >> 3;
                 const bool in = (v >= 0) || nnps_in_fp64<ND>(xi, pi.h, load_pos(d.s.xh, j));
-                if (in && j != i) {
-                    d.s.nbr[(size_t)cnt * N + i] = j;
-                    tm.add(w & 7, cnt);
-                    cnt++;
-                }
+                if (in && j != i) out.add(d, i, w);
             }
         }
     }
-    d.s.nnb[i] = cnt;
-    tm.store(d, i);
+    out.store(d, i);
 }
 
-// The pair records of every list slot, as partisearching stores wij with the
+// The pair records of every list row, as partisearching stores wij with the
 // list (CPP_3-NNPS.cpp:339-345): weight() / weight2() of the pair in FP64, or
-// in FP32 from the FP64 position differences in the bulk form.  One thread per
-// particle walks its list, so for each slot a warp writes consecutive records.
+// in FP32 from the FP64 position differences in the bulk form; for group B
+// the kernel value alone.  One thread per particle walks its list, so for
+// each row a warp writes consecutive values.
+template <int ND, typename R, bool GRAD>
+__device__ __forceinline__ void pairw_rows(const Dev& d, const PairI<R>& I, R rra, int i, int n, int row0, int dir)
+{
+    const ptrdiff_t step = dir * (ptrdiff_t)d.p.N;
+    size_t off = (size_t)row0 * d.p.N + i;
+    const int* p = d.s.nbr + off;
+    if constexpr (sizeof(R) == 8) {
+        // two rows at a time: their chains of dependent FP64 operations
+        // interleave; the next two rows' words are loaded ahead
+        int j0 = (n > 0) ? p[0] >> 3 : i, j1 = (n > 1) ? p[step] >> 3 : i;
+        for (int s = 0; s < n; s += 2) {
+            const Pos pa = load_pos(d.s.xh, j0), pb = load_pos(d.s.xh, j1);
+            p += 2 * step;
+            if (s + 2 < n) j0 = p[0] >> 3;
+            j1 = (s + 3 < n) ? p[step] >> 3 : j0;
+            R wa[4], wb[4];
+            pair_w64<ND, GRAD>(d, I, rra, pa, wa);
+            pair_w64<ND, GRAD>(d, I, rra, pb, wb);
+            if (GRAD) store_g<ND, R>(d, off, wa);
+            store_v<R>(d, off, wa[3]);
+            off += step;
+            if (s + 1 < n) {
+                if (GRAD) store_g<ND, R>(d, off, wb);
+                store_v<R>(d, off, wb[3]);
+            }
+            off += step;
+        }
+        return;
+    }
+    // the next row's index and position are loaded one row ahead
+    Pos pn = load_pos(d.s.xh, (n > 0) ? *p >> 3 : i);
+    p += step;
+    int jn = (n > 1) ? *p >> 3 : 0;
+    for (int s = 0; s < n; s++) {
+        const Pos pj = pn;
+        p += step;
+        if (s + 1 < n) pn = load_pos(d.s.xh, jn);
+        if (s + 2 < n) jn = *p >> 3;
+        R w[4];
+        pair_w_raw<ND, R>(d, I, rra, pj, w);
+        if (GRAD) store_g<ND, R>(d, off, w);
+        store_v<R>(d, off, w[3]);
+        off += step;
+    }
+}
+
 template <int ND, typename R>
 __device__ __forceinline__ void pairw_particle(const Dev& d, int i)
 {
-    const int N = d.p.N, nn = nbr_count(d, i);
     const PairI<R> I = pair_i<ND, R>(d, i);
     const R rra = R(1.0) / I.h;     // RN(1 / h_i), the reciprocal of ra when h_j = h_i
-    // the next slot's index and position are loaded one slot ahead
-    int jn = (nn > 1) ? d.s.nbr[(size_t)N + i] : 0;
-    Pos pn = load_pos(d.s.xh, (nn > 0) ? d.s.nbr[i] : i);
-    for (int s = 0; s < nn; s++) {
-        const Pos pj = pn;
-        if (s + 1 < nn) pn = load_pos(d.s.xh, jn);
-        if (s + 2 < nn) jn = d.s.nbr[(size_t)(s + 2) * N + i];
-        R w[4];
-        pair_w_raw<ND, R>(d, I, rra, pj, w);
-        store_w(d, s, i, w);
-    }
+    const int n = d.s.nab[i];
+    pairw_rows<ND, R, true>(d, I, rra, i, n & 0xff, 0, 1);
+    pairw_rows<ND, R, false>(d, I, rra, i, n >> 8, SPH_NB_CAP - 1, -1);
 }
 
 template <int ND>
@@ -674,17 +682,14 @@ __global__ void __launch_bounds__(128, SPH_MINB_PAIRW) k_pairw(Dev d)
 #endif  // !SPH_BULK32
 
 // ---------------------------------------------------------------------------
-// density(): fluid porosity (:25-54) and continuity (:57-165) -> rho_c.  The
-// porosity loop needs only the kernel values and recomputes them from the
-// neighbours' positions (pair_value); the continuity loop reads the gradients
-// from the pair records.
+// density(): fluid porosity (:25-54) and continuity (:57-165) -> rho_c.
 template <int ND>
 __global__ void __launch_bounds__(128, SPH_MINB_DENS) k_density(Dev d)
 {
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     constexpr int nd = ND;
-    const int ti = d.s.type[i], nn = nbr_count(d, i);
+    const int ti = d.s.type[i];
     const int l = *d.s.step;
     const Pos P = load_pos(d.s.xh, i);
     const double xi[3] = {P.x, P.y, P.z};
@@ -694,16 +699,17 @@ __global__ void __launch_bounds__(128, SPH_MINB_DENS) k_density(Dev d)
         Sum<real> sup, sdown;
         const PairI<real> I = pair_i<ND, real>(d, i);
         const real rra = real(1.0) / I.h;
-        MaskIter it(d, i, type_mask(d, i, 2));
-        int s, j;
-        while (it.next(s, j)) {
-            real w[4];
-            pair_value<ND, real>(d, I, rra, j, s, i, w);
+        RowIter it = rows_b(d, i);
+        int j, tj;
+        size_t o;
+        while (it.next(j, tj, o)) {
+            if (tj != 2) continue;
+            const real w3 = pair_value<ND, real>(d, I, rra, j, o);
             const NV pj = load_nv(d.s.rrho, j);     // (mass, porosity, rho, 1 / rho)
             const real mj = (real)pj.vx, rj = (real)pj.vz;
             const double rrj = pj.m;
-            sup.add(div_rho(mj * (real)pj.vy, rj, rrj) * w[3]);
-            sdown.add(div_rho(mj, rj, rrj) * w[3]);
+            sup.add(div_rho(mj * (real)pj.vy, rj, rrj) * w3);
+            sdown.add(div_rho(mj, rj, rrj) * w3);
         }
         const double up = sup.v(), down = sdown.v();
         if (fabs(down) > 1.0e-7) {
@@ -723,23 +729,23 @@ __global__ void __launch_bounds__(128, SPH_MINB_DENS) k_density(Dev d)
         for (int k = 0; k < 3; k++) vi[k] = d.s.vxp[k * N + i];
         const bool solid = (ti == 2 || ti == 4), fluid = (ti == 1 || ti == 3);
         const bool moving = (ti >= 1 && ti <= 4);
-        // slots of i's own type (not for walls) and, for moving i, wall slots
-        const SlotMask wallm = moving ? type_mask(d, i, 0) : SlotMask{0ull, 0ull};
-        MaskIter it(d, i, (ti != 0 ? type_mask(d, i, ti) : SlotMask{0ull, 0ull}) | wallm);
-        int s, j;
-        while (it.next(s, j)) {
+        // rows of i's own type and walls, for moving i
+        RowIter it = rows_a(d, i);
+        if (!moving) it.left = 0;
+        int j, tj;
+        size_t o;
+        while (it.next(j, tj, o)) {
+            if (tj != ti && tj != 0) continue;
             double vxj[3];
             const NV nj = load_nv(d.s.nv, j);
-            if (!wallm.has(s)) {
+            if (tj == ti) {
                 vxj[0] = nj.vx; vxj[1] = nj.vy; vxj[2] = nj.vz;
-            } else if (moving) {
+            } else {
                 // virtual wall velocity (:89-121)
                 for (int k = 0; k < 3; k++) vxj[k] = wall_vel(d, ti, j, vi, k);
-            } else {
-                continue;
             }
-            real w[4];
-            load_w(d, s, i, w);
+            real w[3];
+            load_g<ND, real>(d, o, w);
             const real mj = (real)nj.m;
             if (solid) {
                 const Pos pj = load_pos(d.s.xh, j);
@@ -776,27 +782,25 @@ __global__ void __launch_bounds__(128, SPH_MINB_DENS) k_density(Dev d)
 
 // Shepard filter (:168-188) reading every neighbour's continuity density
 // (Jacobi order), then the local equation of state (CPP_7-1-eos_CR.cpp:22-43).
-// The pass needs only the kernel values, which it recomputes from the
-// neighbours' positions (pair_value) instead of streaming the 32-byte pair
-// records for them.
 template <int ND>
 __global__ void __launch_bounds__(128, SPH_MINB) k_shepard_eos(Dev d)
 {
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
-    const int ti = d.s.type[i], nn = nbr_count(d, i);
+    const int ti = d.s.type[i];
     Sum<real> sup, sdown;
     const PairI<real> I = pair_i<ND, real>(d, i);
     const real rra = real(1.0) / I.h;
-    MaskIter it(d, i, type_mask(d, i, ti));
-    int s, j;
-    while (it.next(s, j)) {
-        real w[4];
-        pair_value<ND, real>(d, I, rra, j, s, i, w);
+    RowIter it = rows_a(d, i);
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
+        if (tj != ti) continue;
+        const real w3 = pair_value<ND, real>(d, I, rra, j, o);
         const double2 cm = reinterpret_cast<const double2*>(d.s.rho_c)[j];
         const real mj = (real)cm.y;
-        sup.add(mj * w[3]);
-        sdown.add(mj / (real)cm.x * w[3]);
+        sup.add(mj * w3);
+        sdown.add(mj / (real)cm.x * w3);
     }
     const double up = sup.v(), down = sdown.v();
     double r = reinterpret_cast<const double2*>(d.s.rho_c)[i].x;
@@ -839,7 +843,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRAIN) k_strain(Dev d)
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     constexpr int nd = ND;
-    const int ti = d.s.type[i], nn = nbr_count(d, i);
+    const int ti = d.s.type[i];
     const Pos P = load_pos(d.s.xh, i);
     double vi[3];
     for (int k = 0; k < 3; k++) vi[k] = d.s.vxp[k * N + i];
@@ -847,15 +851,18 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRAIN) k_strain(Dev d)
     const bool moving = (ti >= 1 && ti <= 4);
     Sum<real> sup[9], sdown[3];
     Sum<real> scolor;
-    // the velocity-gradient and colour sums over i's own type (not walls,
-    // not type 7) and, for moving i, the walls
-    const SlotMask wallm = moving ? type_mask(d, i, 0) : SlotMask{0ull, 0ull};
-    MaskIter it(d, i, ((ti != 0 && ti != 7) ? type_mask(d, i, ti) : SlotMask{0ull, 0ull}) | wallm);
-    int q, j;
-    while (it.next(q, j)) {
-        const bool same = !wallm.has(q);
+    // the velocity-gradient and colour sums over i's own type and the walls,
+    // for moving i
+    RowIter it = rows_a(d, i);
+    if (!moving) it.left = 0;
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
+        const bool same = tj == ti;
+        if (!same && tj != 0) continue;
         real w[4];
-        load_w(d, q, i, w);
+        load_g<ND, real>(d, o, w);
+        w[3] = load_v<real>(d, o);
         // vxp and m_j / rho_j (the quotient the reference forms per pair,
         // formed once per particle by k_shepard_eos: the same value in FP64;
         // the FP32-bulk form divides its FP32 operands per pair)
@@ -928,15 +935,12 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRAIN) k_strain(Dev d)
     if (ti == 2 || ti == 4 || ti == 0) {
         Sum<real> su1, su2, sd1, sd2;
         Sum<real> sus[6], sdsw;
-        const SlotMask m1 = type_mask(d, i, 1), m3 = type_mask(d, i, 3);
-        MaskIter itg(d, i, m1 | m3 | (ti == 0 ? type_mask(d, i, 2) : SlotMask{0ull, 0ull}));
-        while (itg.next(q, j)) {
-            const int tj = m1.has(q) ? 1 : m3.has(q) ? 3 : 2;
-            real w[4];
-            load_w(d, q, i, w);
+        RowIter itg = rows_b(d, i);
+        while (itg.next(j, tj, o)) {
+            if (!(tj == 1 || tj == 3 || (tj == 2 && ti == 0))) continue;
+            const real w3 = load_v<real>(d, o);
             const NV pm = load_nv(d.s.pmr, j);      // (mass, rho, pre, -)
             const real mj = (real)pm.vx, rj = (real)pm.vy;
-            const real w3 = w[3];
             const real pj_ = (ti == 0 && tj == 2) ? real(0) : (real)pm.vz;
             if (tj == 1) { su1.add(mj * pj_ * w3 / rj); sd1.add(mj * w3 / rj); }
             if (tj == 3) { su2.add(mj * pj_ * w3 / rj); sd2.add(mj * w3 / rj); }
@@ -969,16 +973,16 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_saturation(Dev d)
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err || d.s.type[i] != 2) return;
     const double sitas = d.s.s_sitas[i], sitar = d.s.s_sitar[i], cof = sitas - sitar;
-    const int nn = nbr_count(d, i);
     Sum<real> up, down;
-    for (int s = 0; s < nn; s++) {
-        const int j = d.s.nbr[(size_t)s * N + i];
-        if (d.s.type[j] != 1) continue;
-        real w[4];
-        load_w(d, s, i, w);
+    RowIter it = rows_b(d, i);
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
+        if (tj != 1) continue;
+        const real w3 = load_v<real>(d, o);
         const double mr = d.s.mass[j] / d.s.rho[j];
-        up.add((real)(mr * cof) * w[3]);
-        down.add((real)mr * w[3]);
+        up.add((real)(mr * cof) * w3);
+        down.add((real)mr * w3);
     }
     const double tempup = up.v(), tempdown = down.v();
     const double psatu = d.s.satu[i];
@@ -1330,7 +1334,6 @@ __global__ void __launch_bounds__(128, SPH_MINB_ACCA) k_accel_a(Dev d)
     const bool fluid = (ti == 1 || ti == 3);
     const bool solid = (ti == 2 || ti == 4);
     if (!fluid && !solid) return;
-    const int nn = nbr_count(d, i);
     const double ri = d.s.rho[i];
     const int other = (ti == 1) ? 3 : 1;
     const bool minor = (ti == 1) ? d.p.water_minor : d.p.air_minor;
@@ -1350,14 +1353,16 @@ __global__ void __launch_bounds__(128, SPH_MINB_ACCA) k_accel_a(Dev d)
     double pi_own = 0.0;
     if (ti == 2) pi_own = (1 - poro_s) * (-satu_i * prew_i + (1 - satu_i) * prea_i) / dens_s / dens_s;
     if (ti == 4) pi_own = (-satu_i * prew_i + (1 - satu_i) * prea_i) / ri / ri;
-    // fluid: its own and the other fluid's slots; solid: its own type's
-    MaskIter it(d, i, fluid ? (type_mask(d, i, ti) | type_mask(d, i, other)) : type_mask(d, i, ti));
-    int q, j;
-    while (it.next(q, j)) {
+    // fluid: its own and the other fluid's rows; solid: its own type's
+    RowIter it = rows_a(d, i);
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
+        if (tj != ti && !(fluid && tj == other)) continue;
         const bool f_pair = fluid;
         const bool s_pair = solid;
-        real w[4];
-        load_w(d, q, i, w);
+        real w[3];
+        load_g<ND, real>(d, o, w);
         const SR rj_ = load_sr(d.s.sr, j);
         const real mj = (real)rj_.m;
         real srj[6];
@@ -1460,10 +1465,10 @@ __device__ __noinline__ double drag_beta(int form, double por, double ds, double
 // acceleration.  Out of line, so that its nine sums and the particle's
 // stress operands hold registers only for particles next to a wall.
 template <int ND>
-__device__ __noinline__ void wall_stress_rows(int i, int N, unsigned long long wlo, unsigned long long whi, int ti,
+__device__ __noinline__ void wall_stress_rows(int i, int N, WallRows walls, int ti,
                                               bool fluid, bool tran, bool free_struct,
                                               double ri, double satu_i, const int* nbr,
-                                              const double* nbw, const double* mass, const double* rho,
+                                              const real* nbw, const double* mass, const double* rho,
                                               const double* sb, const double* sig_next, const double* prew,
                                               const double* prea, double rows[3])
 {
@@ -1485,15 +1490,12 @@ __device__ __noinline__ void wall_stress_rows(int i, int N, unsigned long long w
         ab[k] = (real)abd[k];
         abr[k] = (real)(abd[k] / ri / ri);
     }
-    // the wall slots (type 0) of the list, in slot order
-    for (int wd = 0; wd < 2; wd++) {
-      unsigned long long m = wd ? whi : wlo;
-      while (m) {
-        const int q = wd * 64 + __ffsll((long long)m) - 1;
-        m &= m - 1;
-        const int j = nbr[(size_t)q * N + i];
-        real w[4];
-        load_w_raw(nbw, N, q, i, w);
+    // the wall rows of group A, in list order
+    const size_t plane = (size_t)SPH_NB_CAP * N;
+    for (int r = walls.pop(); r >= 0; r = walls.pop()) {
+        const size_t o = (size_t)r * N + i;
+        const int j = nbr[o] >> 3;
+        const real w[3] = {nbw[o], nbw[plane + o], (ND == 3) ? nbw[2 * plane + o] : real(0)};
         const real mj = (real)mass[j], rj = (real)rho[j];
         real abj[6];
         if (free_struct && fluid)
@@ -1512,7 +1514,6 @@ __device__ __noinline__ void wall_stress_rows(int i, int N, unsigned long long w
         tb[2][0].add(mj * (abj[5] + abr[5]) * w[0]);
         tb[2][1].add(mj * (abj[4] + abr[4]) * w[1]);
         tb[2][2].add(mj * (abj[2] + abr[2]) * w[2]);
-      }
     }
     for (int k = 0; k < 3; k++) rows[k] = tb[k][0].v() + tb[k][1].v() + tb[k][2].v();
 }
@@ -1568,7 +1569,7 @@ __global__ void __launch_bounds__(128, LOOP ? SPH_MINB_ACCB2 : SPH_MINB_ACCB1) k
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     constexpr int nd = ND;
-    const int ti = d.s.type[i], nn = nbr_count(d, i);
+    const int ti = d.s.type[i];
     const PairI<real> I = pair_i<ND, real>(d, i);
     const double ri = d.s.rho[i];
     const real riR = (real)ri;
@@ -1603,12 +1604,13 @@ __global__ void __launch_bounds__(128, LOOP ? SPH_MINB_ACCB2 : SPH_MINB_ACCB1) k
     }
     if (ffree) {
         for (int k = 0; k < 3; k++) vnow_i[k] = d.s.vx[k * N + i];
-        MaskIter itw(d, i, type_mask(d, i, 0));
-        int q, j;
-        while (itw.next(q, j)) {
-            if (d.s.matype[j] != 5) continue;
-            real w[4];
-            load_w(d, q, i, w);
+        RowIter itw = rows_a(d, i);
+        int j, tj;
+        size_t o;
+        while (itw.next(j, tj, o)) {
+            if (tj != 0 || d.s.matype[j] != 5) continue;
+            real w[3];
+            load_g<ND, real>(d, o, w);
             double vj[3], sg[3];
             for (int k = 0; k < 3; k++) vj[k] = d.s.interfss[k * N + j];
             const double rj = d.s.rho[j];
@@ -1622,13 +1624,16 @@ __global__ void __launch_bounds__(128, LOOP ? SPH_MINB_ACCB2 : SPH_MINB_ACCB1) k
     // the types it pairs (the reference visits every other pair of different
     // types too, but adds nothing for them); each sum in list order
     if (LOOP == 0) {
-        MaskIter it(d, i, (ti != 7) ? type_mask(d, i, ti) : SlotMask{0ull, 0ull});
-        int q, j;
-        while (it.next(q, j)) {
+        RowIter it = rows_a(d, i);
+        int j, tj;
+        size_t o;
+        while (it.next(j, tj, o)) {
+            if (tj != ti) continue;
             const bool dm_pair = damping;
             const Pos pj = load_pos(d.s.xh, j);
             real w[4];
-            load_w(d, q, i, w);
+            load_g<ND, real>(d, o, w);
+            w[3] = (dm_pair || vdamp) ? load_v<real>(d, o) : real(0);
             const NV nj = load_nv(d.s.nv, j);
             const real mj = (real)nj.m, rj = (real)d.s.rho[j];
             const double xj[3] = {pj.x, pj.y, pj.z};
@@ -1671,14 +1676,13 @@ __global__ void __launch_bounds__(128, LOOP ? SPH_MINB_ACCB2 : SPH_MINB_ACCB1) k
         }
     }
     if (LOOP == 1 && d.p.fli >= 1 && (ti == 1 || ti == 2 || ti == 3)) {
-        const SlotMask m1 = type_mask(d, i, 1);
-        MaskIter it(d, i, (ti == 2) ? (m1 | type_mask(d, i, 3)) : type_mask(d, i, 2));
-        int q, j;
-        while (it.next(q, j)) {
-            const int tj = (ti != 2) ? 2 : m1.has(q) ? 1 : 3;
+        RowIter it = rows_b(d, i);
+        int j, tj;
+        size_t o;
+        while (it.next(j, tj, o)) {
+            if (!((ti == 2) ? (tj == 1 || tj == 3) : (tj == 2))) continue;
             const Pos pj = load_pos(d.s.xh, j);
-            real w[4];
-            load_w(d, q, i, w);
+            const real w3 = load_v<real>(d, o);
             const NV nj = load_nv(d.s.nv, j);
             const NV dj = load_nv(d.s.dr4, j);      // (rho, satu, porosity, cop | f_dens)
             const real mj = (real)nj.m, rj = (real)dj.vx;
@@ -1691,7 +1695,7 @@ __global__ void __launch_bounds__(128, LOOP ? SPH_MINB_ACCB2 : SPH_MINB_ACCB1) k
                 inprod = inprod + dvx[k] * dxk;
             }
             if (inprod < 0) {
-                const real w3 = w[3], ga = (real)d.p.g_acc;
+                const real ga = (real)d.p.g_acc;
                 if (DRAG && d.p.fli > 1 && ((ti == 2 && tj == 1) || (ti == 1 && tj == 2))) {
                     // interact2/3 soil-water drag, m_j / rho_j W beta (v_i - v_j)
                     double mv = 0.0;
@@ -1773,7 +1777,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_ACCB) k_accel_b_tail(Dev d)
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     constexpr int nd = ND;
-    const int ti = d.s.type[i], nn = nbr_count(d, i);
+    const int ti = d.s.type[i];
     const PairI<real> I = pair_i<ND, real>(d, i);
     const double ri = d.s.rho[i];
     double vi[3];
@@ -1792,7 +1796,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_ACCB) k_accel_b_tail(Dev d)
     // boundary_effect_free_struct (CPP_9-4:900-990) for the other flbndy
     // values: a fluid's mirrored stress has its shear components negated
     const bool free_struct = !(tran || d.p.flbndy == 1 || d.p.flbndy == 2);
-    const SlotMask wallm = type_mask(d, i, 0);
+    const WallRows walls = wall_rows(d, i);
     // the artificial-viscosity, drag and damping sums of k_accel_b
     double tav[3], tin[3], tdm[3];
     for (int k = 0; k < 3; k++) {
@@ -1804,18 +1808,20 @@ __global__ void __launch_bounds__(128, SPH_MINB_ACCB) k_accel_b_tail(Dev d)
     // line (its nine sums take registers only there); each sum still runs
     // over the list in order
     double tbrow[3] = {0.0, 0.0, 0.0};
-    if (moving && wallm.any())
-        wall_stress_rows<ND>(i, N, wallm.lo, wallm.hi, ti, fluid, tran, free_struct, ri, satu_i, d.s.nbr, d.s.nbw,
-                             d.s.mass, d.s.rho, d.s.sb, d.s.sig_next, d.s.prew, d.s.prea, tbrow);
+    if (moving && walls.any())
+        wall_stress_rows<ND>(i, N, walls, ti, fluid, tran, free_struct, ri, satu_i, d.s.nbr,
+                             reinterpret_cast<const real*>(d.s.nbw), d.s.mass, d.s.rho, d.s.sb, d.s.sig_next, d.s.prew, d.s.prea, tbrow);
     // the artificial-stress pair sum (ART), likewise in a loop of its own
     Sum<real> tu[3];
     if (art) {
-        MaskIter ita(d, i, type_mask(d, i, 2));
-        int q, j;
-        while (ita.next(q, j)) {
+        RowIter ita = rows_a(d, i);
+        int j, tj;
+        size_t o;
+        while (ita.next(j, tj, o)) {
+            if (tj != 2) continue;
             const Pos pj = load_pos(d.s.xh, j);
-            real w[4];
-            load_w(d, q, i, w);
+            real w[3];
+            load_g<ND, real>(d, o, w);
             const real mj = (real)d.s.mass[j];
             const double xj[3] = {pj.x, pj.y, pj.z};
             // artificial_stress_2d/_3d pair sum (CPP_9-5-artificialstress.cpp:
@@ -2011,7 +2017,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_XSPH) k_xsph_update(Dev d)
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     constexpr int nd = ND;
-    const int ti = d.s.type[i], nn = nbr_count(d, i);
+    const int ti = d.s.type[i];
     const double dt = step_dt(d);
     const PairI<real> I = pair_i<ND, real>(d, i);
     double vm[3];
@@ -2021,25 +2027,26 @@ __global__ void __launch_bounds__(128, SPH_MINB_XSPH) k_xsph_update(Dev d)
     }
     const bool moving = (ti >= 1 && ti <= 4);
     double vn[3] = {vm[0], vm[1], vm[2]};
-    const SlotMask wallm = type_mask(d, i, 0);
-    const bool any_wall = wallm.any();
+    WallRows walls = wall_rows(d, i);
+    const bool any_wall = walls.any();
     if (d.p.if_move != 2 && moving) {
         const real xs_same = (real)((ti == 1) ? d.p.xsph0 : (ti == 3) ? d.p.xsph2 : d.p.xsph1);
         const real xs_wall = (real)((ti == 1 || ti == 3) ? 0.006 : d.p.xsph1 / 5.0);
         Sum<real> stu[3], sdown;
-        // same-type and wall slots in list order (disjoint for moving i)
-        MaskIter it(d, i, type_mask(d, i, ti) | wallm);
-        int q, j;
-        while (it.next(q, j)) {
-            const real xishu = wallm.has(q) ? xs_wall : xs_same;
-            real w[4];
-            load_w(d, q, i, w);
+        // same-type and wall rows in list order
+        RowIter it = rows_a(d, i);
+        int j, tj;
+        size_t o;
+        while (it.next(j, tj, o)) {
+            if (tj != ti && tj != 0) continue;
+            const real xishu = (tj == 0) ? xs_wall : xs_same;
+            const real w3 = load_v<real>(d, o);
             const NV nj = load_nv(d.s.vx_next, j);
             const real mj = (real)nj.m, rj = (real)d.s.rho[j];
             const double vjs[3] = {nj.vx, nj.vy, nj.vz};
             for (int k = 0; k < nd; k++)
-                stu[k].add(xishu * mj * (real)(vjs[k] - vm[k]) * w[3] / rj);
-            sdown.add(mj * w[3] / rj);
+                stu[k].add(xishu * mj * (real)(vjs[k] - vm[k]) * w3 / rj);
+            sdown.add(mj * w3 / rj);
         }
         double tu[3];
         for (int k = 0; k < 3; k++) tu[k] = stu[k].v();
@@ -2057,9 +2064,8 @@ __global__ void __launch_bounds__(128, SPH_MINB_XSPH) k_xsph_update(Dev d)
     if (vcorr && any_wall) {
         const double a = (d.p.flbndy == 1) ? 0.30 : d.p.coe_bndy, b = a, dr = d.p.dr;
         double tb[3] = {0, 0, 0};
-        MaskIter itw(d, i, wallm);
-        int q, j;
-        while (itw.next(q, j)) {
+        for (int r = walls.pop(); r >= 0; r = walls.pop()) {
+            const int j = d.s.nbr[(size_t)r * N + i] >> 3;
             const Pos pj = load_pos(d.s.xh, j);
             const double xj[3] = {pj.x, pj.y, pj.z};
             double inprod = 0.0, dst = 0.0;
@@ -2152,15 +2158,14 @@ __global__ void __launch_bounds__(128) k_tm_vb(Dev d)
     if (i >= N || *d.s.err) return;
     const int ti = d.s.type[i];
     if (ti == 0 || ti == 7) return;
-    const int nn = nbr_count(d, i);
     int ids[SPH_NB_CAP];
     double dsts[SPH_NB_CAP];
     // without such a wall the reference reads particle 0 (of the instance)
     int total = 0, id = d.s.o2i[(d.p.ninst > 0) ? d.s.inst[d.s.pinst[i]].first : 0];
     const Pos P = load_pos(d.s.xh, i);
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        if (d.s.type[j] != 0) continue;
+    WallRows walls = wall_rows(d, i);
+    for (int r = walls.pop(); r >= 0; r = walls.pop()) {
+        const int j = d.s.nbr[(size_t)r * N + i] >> 3;
         const Pos pj = load_pos(d.s.xh, j);
         const double d2 = (P.x - pj.x) * (P.x - pj.x) + (P.y - pj.y) * (P.y - pj.y) + (P.z - pj.z) * (P.z - pj.z);
         ids[total] = j;
@@ -2245,16 +2250,14 @@ __global__ void __launch_bounds__(128) k_tm_wall(Dev d)
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     if (d.s.type[i] != 0) return;
-    const int nn = nbr_count(d, i);
     double up[4][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, down[4] = {0, 0, 0, 0};
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        const int tj = d.s.type[j];
+    RowIter it = rows_b(d, i);
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
         if (tj < 1 || tj > 4) continue;
         const int p = tj - 1;
-        real w[4];
-        load_w(d, q, i, w);
-        const double w3 = w[3], mj = d.s.mass[j], rj = d.s.rho[j];
+        const double w3 = load_v<real>(d, o), mj = d.s.mass[j], rj = d.s.rho[j];
         up[p][0] = up[p][0] + mj * d.s.vel_bndy[j] * w3 / rj;
         up[p][1] = up[p][0] + mj * d.s.vel_bndy[(size_t)N + j] * w3 / rj;
         up[p][2] = up[p][0] + mj * d.s.vel_bndy[(size_t)2 * N + j] * w3 / rj;
@@ -2311,16 +2314,19 @@ __global__ void __launch_bounds__(128) k_ss_pair(Dev d)
     for (int q = 0; q < 3; q++) d.s.ss_id[(size_t)q * N + i] = -1;
     const int ti = d.s.type[i];
     if (!(ti == 1 || ti == 2)) return;
-    const int form = d.p.ss_type, nn = nbr_count(d, i);
+    const int form = d.p.ss_type;
     const double dt = step_dt(d), dr = d.p.dr, myu = d.p.ss_myu, zeta = d.p.ss_zeta;
     const double reach = (form == 1) ? 0.5 * dr : dr;
     int ids[SPH_NB_CAP];
     double dsts[SPH_NB_CAP];
     int total = 0;
     const SSPt p4 = ss_pt(d, i);
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        if (d.s.type[j] != 4) continue;
+    // structure particles: solids share their group with them, fluids do not
+    RowIter it = (ti == 2) ? rows_a(d, i) : rows_b(d, i);
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
+        if (tj != 4) continue;
         const SSPt pj = ss_pt(d, j);
         const double dd = (p4.x - pj.x) * (p4.x - pj.x) + (p4.y - pj.y) * (p4.y - pj.y) + (p4.z - pj.z) * (p4.z - pj.z);
         ids[total] = j;
@@ -2508,25 +2514,29 @@ __global__ void __launch_bounds__(128) k_ss_struct(Dev d)
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     if (d.s.type[i] != 4) return;
-    const int nn = nbr_count(d, i);
     int src[SPH_NB_CAP], srco[SPH_NB_CAP], slot[SPH_NB_CAP];
     int m = 0;
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        const int tj = d.s.type[j];
-        if (!(tj == 1 || tj == 2)) continue;
-        for (int s = 0; s < 3; s++)
-            if (d.s.ss_id[(size_t)s * N + j] == i) {
-                // insertion by source index in the caller's order
-                const int jo = d.s.i2o[j];
-                int p = m++;
-                while (p > 0 && srco[p - 1] > jo) {
-                    src[p] = src[p - 1]; srco[p] = srco[p - 1]; slot[p] = slot[p - 1]; p--;
+    // soil (group A), then water (group B): the order below does not depend on
+    // the list's
+    for (int pass = 0; pass < (d.p.split ? 2 : 1); pass++) {
+        RowIter it = pass ? rows_b(d, i) : rows_a(d, i);
+        int j, tj;
+        size_t o;
+        while (it.next(j, tj, o)) {
+            if (!(tj == 1 || tj == 2)) continue;
+            for (int s = 0; s < 3; s++)
+                if (d.s.ss_id[(size_t)s * N + j] == i) {
+                    // insertion by source index in the caller's order
+                    const int jo = d.s.i2o[j];
+                    int p = m++;
+                    while (p > 0 && srco[p - 1] > jo) {
+                        src[p] = src[p - 1]; srco[p] = srco[p - 1]; slot[p] = slot[p - 1]; p--;
+                    }
+                    src[p] = j;
+                    srco[p] = jo;
+                    slot[p] = s;
                 }
-                src[p] = j;
-                srco[p] = jo;
-                slot[p] = s;
-            }
+        }
     }
     double f[6] = {0, 0, 0, 0, 0, 0};
     for (int e = 0; e < m; e++)
@@ -2548,7 +2558,6 @@ __global__ void __launch_bounds__(128) k_tran_wall(Dev d)
     if (i >= N || *d.s.err) return;
     if (d.s.type[i] != 0) return;
     const bool free_slip = d.p.flbndy == 4 || d.p.flbndy == 14;
-    const int nn = nbr_count(d, i);
     const Pos P = load_pos(d.s.xh, i);
     const double dr = d.p.dr;
     double us[4][6], uv[4][3], down[4];
@@ -2557,14 +2566,13 @@ __global__ void __launch_bounds__(128) k_tran_wall(Dev d)
         for (int k = 0; k < 3; k++) uv[p][k] = 0.0;
         down[p] = 0.0;
     }
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        const int tj = d.s.type[j];
+    RowIter it = rows_b(d, i);
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
         if (tj < 1 || tj > 4) continue;
         const int p = tj - 1;
-        real wr[4];
-        load_w(d, q, i, wr);
-        const double w3 = wr[3], mj = d.s.mass[j], rj = d.s.rho[j];
+        const double w3 = load_v<real>(d, o), mj = d.s.mass[j], rj = d.s.rho[j];
         double sj[6], vj[3];
         for (int k = 0; k < 6; k++) sj[k] = d.s.sig_next[(size_t)k * N + j];
         for (int k = 0; k < 3; k++) vj[k] = d.s.vx_vb[(size_t)k * N + j];
@@ -2611,15 +2619,14 @@ __global__ void __launch_bounds__(128) k_free_solid(Dev d)
     d.s.fsol_on[i] = 0;
     const int ti = d.s.type[i];
     if (ND == 2 && !(ti >= 1 && ti <= 4)) return;
-    const int nn = nbr_count(d, i);
     const double dt = step_dt(d), dr = d.p.dr, myu = d.p.ss_myu, zeta = d.p.ss_zeta;
     int ids[SPH_NB_CAP];
     double dsts[SPH_NB_CAP];
     int total = 0;
     const SSPt p4 = ss_pt(d, i);
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        if (d.s.type[j] != 0) continue;
+    WallRows walls = wall_rows(d, i);
+    for (int r = walls.pop(); r >= 0; r = walls.pop()) {
+        const int j = d.s.nbr[(size_t)r * N + i] >> 3;
         const SSPt pj = ss_pt(d, j);
         const double dd = (p4.x - pj.x) * (p4.x - pj.x) + (p4.y - pj.y) * (p4.y - pj.y) + (p4.z - pj.z) * (p4.z - pj.z);
         ids[total] = j;
@@ -2757,19 +2764,19 @@ __global__ void __launch_bounds__(128) k_coupled(Dev d)
     if (i >= N || *d.s.err) return;
     const int ti = d.s.type[i];
     if (!(ti == 4 || ti == 2 || ti == 1)) return;
-    const int nn = nbr_count(d, i);
     double si[6];
     for (int k = 0; k < 6; k++) si[k] = d.s.sig_next[(size_t)k * N + i];
     const double ri = d.s.rho[i];
     double tu[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        const int tj = d.s.type[j];
+    RowIter it = rows_a(d, i);         // the whole list: these runs do not split it
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
         const bool plus = (ti == 4 && tj == 2) || (ti == 2 && tj == 4) || (ti == 4 && tj == 1);
         const bool minus = (ti == 1 && tj == 4);
         if (!(plus || minus)) continue;
-        real wr[4];
-        load_w(d, q, i, wr);
+        real wr[3];
+        load_g<3, real>(d, o, wr);
         const double w[3] = {wr[0], wr[1], wr[2]};
         const double mj = d.s.mass[j], rj = d.s.rho[j];
         double sj[6], a[6], b[6];
@@ -2876,19 +2883,19 @@ __device__ __forceinline__ void kgc_particle(const Dev& d, int i)
 {
     const int N = d.p.N;
     const int ti = d.s.type[i];
-    const int nn = nbr_count(d, i);
     const Pos P = load_pos(d.s.xh, i);
     const double xi[3] = {P.x, P.y, P.z};
     double L[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        const int tj = d.s.type[j];
+    RowIter it = rows_a(d, i);
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
         const bool take = (ti == 2 && (tj == 2 || tj == 0 || tj == 4)) || (ti == 4 && (tj == 4 || tj == 0 || tj == 2));
         if (!take) continue;
         const Pos pj = load_pos(d.s.xh, j);
         const double xj[3] = {pj.x, pj.y, pj.z};
-        R wr[4];
-        load_w(d, q, i, wr);
+        R wr[3];
+        load_g<ND, R>(d, o, wr);
         const double w[3] = {wr[0], wr[1], wr[2]};
         const double mr = d.s.mass[j] / d.s.rho[j];
         double xij[3];
@@ -2925,14 +2932,16 @@ __device__ __forceinline__ void kgc_particle(const Dev& d, int i)
     R a[9];
     for (int r = 0; r < 3; r++)
         for (int c = 0; c < 3; c++) a[r * 3 + c] = (R)B[r][c];
-    for (int q = 0; q < nn; q++) {
-        R w[4];
-        load_w(d, q, i, w);
+    const int na = d.s.nab[i] & 0xff;
+    for (int r = 0; r < na; r++) {
+        R w[3];
+        o = (size_t)r * N + i;
+        load_g<ND, R>(d, o, w);
         const R c0 = a[0] * w[0] + a[1] * w[1] + a[2] * w[2];
         const R c1 = a[3] * w[0] + a[4] * w[1] + a[5] * w[2];
         const R c2 = a[6] * w[0] + a[7] * w[1] + a[8] * w[2];
         w[0] = c0; w[1] = c1; w[2] = c2;
-        store_w(d, q, i, w);
+        store_g<ND, R>(d, o, w);
     }
 }
 
@@ -2962,14 +2971,14 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_regu(Dev d, const double* src
         for (int k = 0; k < 6; k++) dst[(size_t)k * N + i] = zero ? 0.0 : src[(size_t)k * N + i];
         return;
     }
-    const int ti = d.s.type[i], nn = nbr_count(d, i);
+    const int ti = d.s.type[i];
     double up[6] = {0, 0, 0, 0, 0, 0}, down = 0.0;
-    for (int q = 0; q < nn; q++) {
-        const int j = d.s.nbr[(size_t)q * N + i];
-        if (d.s.type[j] != ti) continue;
-        real wr[4];
-        load_w(d, q, i, wr);
-        const double w3 = wr[3];
+    RowIter it = rows_a(d, i);
+    int j, tj;
+    size_t o;
+    while (it.next(j, tj, o)) {
+        if (tj != ti) continue;
+        const double w3 = load_v<real>(d, o);
         const double mr = d.s.mass[j] / d.s.rho[j];
         for (int k = 0; k < 6; k++) up[k] = up[k] + mr * w3 * (zero ? 0.0 : src[(size_t)k * N + j]);
         down = down + mr * w3;
@@ -3093,9 +3102,9 @@ static_assert(sizeof(sphk_stage_names) / sizeof(sphk_stage_names[0]) == SPHK_NST
 // correction; returns the number of this library's kernels it launched
 #if SPHGPU_CHECK
 // The bounds-checked build (SPHGPU_CHECK=1): after the search, every index the
-// later passes take from it is checked -- each list slot holds a particle
-// other than i within [0, N), the slot masks mark exactly the slots of their
-// type, the sorted order is a permutation and the cell ranges stay within the
+// later passes take from it is checked -- each list row holds a particle
+// other than i within [0, N) with its type code, in the group of that type, the
+// wall rows mark exactly the walls, the sorted order is a permutation and the cell ranges stay within the
 // sorted positions.  A violation sets the error word to SPH_ERR_CHECK (the
 // passes after it then return at once) instead of trapping.
 __global__ void k_check_lists(Dev d)
@@ -3103,18 +3112,19 @@ __global__ void k_check_lists(Dev d)
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     bool bad = false;
-    const int nn = nbr_count(d, i);
-    if (nn < 0 || nn > SPH_NB_CAP) bad = true;
+    const int na = d.s.nab[i] & 0xff, nb = d.s.nab[i] >> 8;
+    if (na + nb > SPH_NB_CAP || na + nb > d.s.nnb[i]) bad = true;
     const int q = d.s.sortpos[i];
     if (q < 0 || q >= N || d.s.pid_sorted[q] != i) bad = true;
-    for (int s = 0; s < nn && !bad; s++) {
-        const int j = d.s.nbr[(size_t)s * N + i];
+    const Groups g = list_groups(d, d.s.type[i]);
+    const WallRows walls = wall_rows(d, i);
+    for (int s = 0; s < na + nb && !bad; s++) {
+        const int w = d.s.nbr[(size_t)(s < na ? s : SPH_NB_CAP - 1 - (s - na)) * N + i], j = w >> 3, t = w & 7;
         if (j < 0 || j >= N || j == i) { bad = true; break; }
         const int tj = d.s.type[j];
-        for (int t = 0; t <= 4; t++) {
-            const SlotMask m = type_mask(d, i, t);
-            if (m.has(s) != (tj == t)) bad = true;
-        }
+        if (t != ((tj >= 0 && tj <= 4) ? tj : 7)) bad = true;
+        if (!(((s < na ? g.a : g.b) >> t) & 1u)) bad = true;
+        if (s < na && (((s < 64 ? walls.lo >> s : walls.hi >> (s - 64)) & 1ull) != 0) != (t == 0)) bad = true;
     }
     const int c = d.s.cell[i];
     if (c >= 0 && c < d.p.ctotal + 4) {
