@@ -931,7 +931,7 @@ sphgpu_ctx* sphgpu_create(const sphgpu_params* P, int device)
     r |= dalloc(c, &s.s_c, N); r |= dalloc(c, &s.s_fs, N);
     r |= dalloc(c, &s.s_ann, N); r |= dalloc(c, &s.s_zmf, N); r |= dalloc(c, &s.s_ramda, N); r |= dalloc(c, &s.s_sme0, N);
     r |= dalloc(c, &s.s_yalf, N); r |= dalloc(c, &s.s_ykap, N); r |= dalloc(c, &s.s_yalf_dil, N);
-    r |= dalloc(c, &s.xh, 4 * (size_t)N); r |= dalloc(c, &s.xh_next, 4 * (size_t)N); r |= dalloc(c, &s.xs, 4 * (size_t)N); r |= dalloc(c, &s.xsf, 4 * (size_t)N);
+    r |= dalloc(c, &s.xh, 4 * (size_t)N); r |= dalloc(c, &s.xh_next, 4 * (size_t)N); r |= dalloc(c, &s.xs, 4 * (size_t)N); r |= dalloc(c, &s.xsf, 4 * (size_t)N); r |= dalloc(c, &s.xsp, 3 * (size_t)SPH_XSP_STRIDE(N));
     r |= dalloc(c, &s.de, 6 * (size_t)N); r |= dalloc(c, &s.we, 6 * (size_t)N); r |= dalloc(c, &s.color, N);
     r |= dalloc(c, &s.sr, 8 * (size_t)N);
     r |= dalloc(c, &s.eps_tmp, 6 * (size_t)N); r |= dalloc(c, &s.sig_tmp, 6 * (size_t)N);
@@ -954,9 +954,9 @@ sphgpu_ctx* sphgpu_create(const sphgpu_params* P, int device)
     r |= dalloc(c, &s.val_in, N); r |= dalloc(c, &s.pid_sorted, N);
     r |= dalloc(c, &s.cstart, M); r |= dalloc(c, &s.cend, M);
     r |= dalloc(c, &s.nnb, N); r |= dalloc(c, &s.nbr, (size_t)SPH_NB_CAP * N);
-    r |= dalloc(c, &s.nps, N); r |= dalloc(c, &s.sortpos, N); r |= dalloc(c, &s.pts, N);
+    r |= dalloc(c, &s.nps, N); r |= dalloc(c, &s.sortpos, N);
     if (!s.accb) r |= dalloc(c, &s.accb, 9 * (size_t)N);   // (19N when alloc_optional sized it for vibration)
-    r |= dalloc(c, &s.nbrs, (size_t)SPH_NB_CAP * N);
+    r |= dalloc(c, &s.nbrs, (size_t)SPH_NBRS_ROW * N);
     r |= dalloc(c, &s.nab, N); r |= dalloc(c, &s.nbm, 2 * (size_t)N);
     r |= dalloc(c, &s.nbw, 4 * (size_t)SPH_NB_CAP * N);
     r |= dalloc(c, &s.err, 1); r |= dalloc(c, &s.step, 1);

@@ -36,6 +36,10 @@
 #include <cstdint>
 
 #define SPH_NB_CAP 99          // Par_Cell::influ[100], slots 1..99 (Class_NNPS.h:71)
+#define SPH_NBRS_ROW 108       // words of a provisional list: 99 in two groups, each rounded up to 4
+// values per plane of the search's position planes: whole lines, and room to
+// read up to 35 positions past the last
+#define SPH_XSP_STRIDE(N) (((N) + 36 + 63) / 64 * 64)
 #define SPH_ERR_CELL 3         // parttocell, CPP_3-NNPS.cpp:247-257
 #define SPH_ERR_NEIGH 5        // partisearching, CPP_3-NNPS.cpp:313-319
 #define SPHK_NSTAGES 21        // entries of sphk_stage_names (one event bracket each)
@@ -137,7 +141,9 @@ struct DevState {
     // positions (x, y, z, h) records, ping-pong
     double *xh, *xh_next;
     double *xs;                // xh in cell-sorted order (NNPS scan)
-    float *xsf;                // xs as FP32 (x - xmin, y - ymin, z - zmin, h) records: the NNPS prefilter
+    float *xsf;                // xs as FP32 records (x - xmin, y - ymin, z - zmin, word), word the particle
+                               // index << 3 | its type code (the type for types 0-4, else 7) as bits
+    float *xsp;                // its x, y, z as planes of SPH_XSP_STRIDE(N) values: the scan's tests
     // dynamic state
     double *vx;                // velocity after the step
     double *vx_next;           // per particle (vx x, y, z before XSPH, mass): one 32-byte record
@@ -201,12 +207,10 @@ struct DevState {
     int *val_in, *pid_sorted;
     int *cstart, *cend;        // [ctotal + 4]
     int *nnb;                  // neighbour count (may exceed the cap: error 5)
-    // the neighbour search by cell-sorted position q: pts[q] = the particle
-    // index << 3 | its type code (the type for types 0-4, else 7); the scan's
-    // provisional count (-1: the particle takes the direct FP64 search) and
-    // provisional list nbrs[s * N + q] of candidates' pts words (~word for a
-    // candidate within the FP32 margin of the radius); sortpos[i] = q
-    int *nps, *nbrs, *sortpos, *pts;
+    // the neighbour search by cell-sorted position q: the scan's group sizes
+    // nps[q] (as nab) and lists of index-and-type words, nbrs (k_nnps);
+    // sortpos[i] = q
+    int *nps, *nbrs, *sortpos;
     // the momentum pass's artificial-viscosity, drag and damping sums, from
     // its loop kernel to its tail kernel: accb[(3 g + k) * N + i] (9N); with
     // vibration (flv != 0) also the free-field sums of the walls (g = 3) and

@@ -9,8 +9,9 @@
 //   radix sort     Binary_Sort's order: cell ascending, index descending
 //   k_cellreset    cell_info reset                              (CPP_3-NNPS.cpp:196-201)
 //   k_cellrange    cell_info start/end (:621-629) + the cell-sorted copy of positions
-//   k_nnps         partisearching: stencil scan in cell-sorted order, FP32 prefilter
-//   k_nnps_resolve FP64 decisions of the undecided candidates, neighbour list, slot masks
+//   k_nnps         partisearching: stencil scan in cell-sorted order, FP32 prefilter,
+//                  FP64 decisions of the undecided candidates
+//   k_pairw        neighbour lists and pair records in the held order
 //   k_density      fluid porosity + continuity                  (CPP_6-density.cpp:25-165)
 //   k_shepard_eos  Shepard filter (Jacobi) + local EOS          (CPP_6-density.cpp:168-188, CPP_7-1-eos_CR.cpp:22-43)
 //   k_strain       velocity gradient, strain rate and spin, gathered pore pressures and
@@ -80,6 +81,9 @@ namespace SPH_NS {
 #endif
 #ifndef SPH_MINB_ACCB2
 #define SPH_MINB_ACCB2 7
+#endif
+#ifndef SPH_MINB_NNPS
+#define SPH_MINB_NNPS 7
 #endif
 #ifndef SPH_MINB_PAIRW
 #define SPH_MINB_PAIRW SPH_MINB
@@ -332,11 +336,19 @@ __global__ void k_cellrange(Dev d)
     }
     d.s.sortpos[pid] = q;
     const int t = d.s.type[pid];
-    d.s.pts[q] = (pid << 3) | ((t >= 0 && t <= 4) ? t : 7);
+    const int w = (pid << 3) | ((t >= 0 && t <= 4) ? t : 7);
     const Pos r = load_pos(d.s.xh, pid);
     store_pos(d.s.xs, q, r);
-    reinterpret_cast<float4*>(d.s.xsf)[q] =
-        make_float4((float)(r.x - g.xmin), (float)(r.y - g.ymin), (float)(r.z - g.zmin), (float)r.h);
+    // the search's FP32 records with the index-and-type word, and its planes;
+    // a candidate whose h is not dr has NaN for x, which no bound decides, so
+    // it takes the FP64 test
+    float4 f = make_float4((float)(r.x - g.xmin), (float)(r.y - g.ymin), (float)(r.z - g.zmin), __int_as_float(w));
+    if ((float)r.h != (float)d.p.dr) f.x = __int_as_float(0x7fffffff);
+    reinterpret_cast<float4*>(d.s.xsf)[q] = f;
+    const size_t NP = (size_t)SPH_XSP_STRIDE(N);
+    d.s.xsp[q] = f.x;
+    d.s.xsp[NP + q] = f.y;
+    d.s.xsp[2 * NP + q] = f.z;
 }
 
 // partisearching (CPP_3-NNPS.cpp:265-374): neighbours of i in stencil order,
@@ -373,121 +385,17 @@ __device__ __forceinline__ bool nnps_in_fp64(const double xi[3], double hi, cons
     return sqrt(d2) <= T;
 }
 
-// FP32 prefilter of the candidates of one particle: its (x - xmin, y - ymin,
-// z - zmin, h) in FP32, the margin terms, and the decision bounds lo / hi of a
-// candidate with the same h (the usual case), so that such a candidate costs
-// its squared distance and two comparisons.  The squared distance is summed
-// with fused multiply-adds: one rounding per term instead of two, inside the
-// margin derived for separate roundings.
-struct Prefilter {
-    float fx, fy, fz, fh, ce, ct, lo0, hi0;
-};
-
+// The decision bounds of a particle's candidates, all of h equal to its own:
+// inside below lo, outside above hi, in FP64 between.
 template <int ND>
-__device__ __forceinline__ void prefilter_bounds(const Prefilter& P, float hj, float* lo, float* hi)
+__device__ __forceinline__ void prefilter_bounds(float fh, float ce, float* lo, float* hi)
 {
     constexpr float U = 5.9604645e-8f;     // 2^-24
-    const float Tf = P.fh + hj, T2f = Tf * Tf;
-    const float e = P.ce + 4.4f * U * Tf;
-    const float M = ND * e * (4.f * Tf + e) + P.ct * T2f;
+    const float Tf = fh + fh, T2f = Tf * Tf;
+    const float e = ce + 4.4f * U * Tf;
+    const float M = ND * e * (4.f * Tf + e) + 32.f * U * T2f;
     *lo = T2f - M;
     *hi = T2f + M;
-}
-
-template <int ND>
-__device__ __forceinline__ Prefilter make_prefilter(float fx, float fy, float fz, float fh, float ce, float ct)
-{
-    Prefilter P{fx, fy, fz, fh, ce, ct, 0.f, 0.f};
-    prefilter_bounds<ND>(P, fh, &P.lo0, &P.hi0);
-    return P;
-}
-
-// verdict of one candidate: 1 inside, 0 outside, -1 undecided (within the
-// rounding margin of the radius).  A candidate beyond twice the radius is
-// outside; hi < 4 T^2, so the bounds test covers that case too.
-template <int ND>
-__device__ __forceinline__ int nnps_prefilter(const Prefilter& P, float4 fj)
-{
-    float t = P.fx - fj.x;
-    float d2f = t * t;
-    t = P.fy - fj.y;
-    d2f = __fmaf_rn(t, t, d2f);
-    if (ND == 3) {
-        t = P.fz - fj.z;
-        d2f = __fmaf_rn(t, t, d2f);
-    }
-    float lo = P.lo0, hi = P.hi0;
-    if (fj.w != P.fh) {
-        const float Tf = P.fh + fj.w;
-        if (d2f > 4.f * (Tf * Tf)) return 0;
-        prefilter_bounds<ND>(P, fj.w, &lo, &hi);
-    }
-    if (d2f < lo) return 1;
-    if (d2f > hi) return 0;
-    return -1;
-}
-
-// One particle's list as it is built: the rows of its two groups and the wall
-// rows of group A, in list order
-struct ListOut {
-    Groups g;
-    int cnt, na, nb;               // neighbours (of every type), rows of A and B
-    unsigned long long lo, hi;
-    __device__ __forceinline__ ListOut(const Dev& d, int t) : g(list_groups(d, t)), cnt(0), na(0), nb(0), lo(0ull), hi(0ull) {}
-    // word w = index << 3 | type code; past the capacity it is only counted
-    __device__ __forceinline__ void add(const Dev& d, int i, int w)
-    {
-        const int t = w & 7;
-        cnt++;
-        if (cnt > SPH_NB_CAP) return;
-        if ((g.a >> t) & 1u) {
-            if (t == 0) {
-                if (na < 64) lo |= 1ull << na;
-                else hi |= 1ull << (na - 64);
-            }
-            d.s.nbr[(size_t)na * d.p.N + i] = w;
-            na++;
-        } else if ((g.b >> t) & 1u) {
-            d.s.nbr[(size_t)(SPH_NB_CAP - 1 - nb) * d.p.N + i] = w;
-            nb++;
-        }
-    }
-    __device__ __forceinline__ void store(const Dev& d, int i) const
-    {
-        d.s.nnb[i] = cnt;
-        d.s.nab[i] = na | (nb << 8);
-        d.s.nbm[i] = lo;
-        d.s.nbm[(size_t)d.p.N + i] = hi;
-    }
-};
-
-// partisearching with every candidate decided in FP64 as soon as it is met
-// (used when the FP32 prefilter does not apply to the particle, or when its
-// provisional list below overflows)
-template <int ND>
-__device__ __forceinline__ void nnps_direct(const Dev& d, int i, int nc, const Pos& pi, bool fast, const Prefilter& P,
-                                            ListOut& out)
-{
-    constexpr int nst = (ND == 2) ? 9 : 27;
-    const double xi[3] = {pi.x, pi.y, pi.z};
-    const float4* xsf = reinterpret_cast<const float4*>(d.s.xsf);
-    const CellGrid g = cell_grid(d, i);
-    for (int nj = 0; nj < nst; nj++) {
-        const int nl = cell_link<ND>(g, nc, nj);
-        if (nl <= 0) continue;
-        const int start = d.s.cstart[nl], end = d.s.cend[nl];
-        for (int q = start; q <= end; q++) {
-            int v = fast ? nnps_prefilter<ND>(P, xsf[q]) : -1;
-            if (v < 0) v = nnps_in_fp64<ND>(xi, pi.h, load_pos(d.s.xs, q)) ? 1 : 0;
-            if (v) {
-                const int w = d.s.pts[q];
-                if (i != (w >> 3)) {
-                    out.add(d, i, w);
-                    if (out.cnt > SPH_NB_CAP) raise_err(d.s.err, SPH_ERR_NEIGH);
-                }
-            }
-        }
-    }
 }
 
 // partisearching (CPP_3-NNPS.cpp:265-374): neighbours of i in stencil order,
@@ -508,95 +416,220 @@ __device__ __forceinline__ void nnps_direct(const Dev& d, int i, int nc, const P
 //
 // Two passes.  The scan (k_nnps) runs one thread per cell-sorted position,
 // so the lanes of a warp belong to one or two cells, walk the same stencil
-// cells and load the same candidate records (one broadcast per load instead
-// of a line per lane).  It stores, in candidate order, the index-and-type
-// word w of each candidate inside (w) or undecided (~w) into the provisional
-// list of its own sorted position, nbrs[s * N + q], which the lanes of a warp
-// fill row by row.  The resolve pass (k_nnps_resolve) runs one thread per
-// particle in the caller's order: it reads its provisional list, decides the
-// undecided candidates in FP64, and writes the list into its two groups.  The
-// order within a group is the one a single pass in candidate order gives.  A provisional list
-// longer than the capacity (possible only when undecided candidates or the
-// particle itself push it over), and a particle the FP32 test does not apply
-// to, are searched again by the direct form, which also raises the
-// reference's error for a true overflow.
-template <int ND>
-__global__ void __launch_bounds__(128, SPH_MINB) k_nnps(Dev d)
+// cells and load the same candidate records.  It works in two parts.  The
+// first tests the candidates of every stencil cell, four per load of the
+// planes xsp with packed FP32 arithmetic, and keeps one bit per candidate
+// that is not outside (shared memory, a word per cell and thread).  The second
+// visits the set bits in order: a candidate that is undecided takes the FP64
+// test, and a neighbour's index-and-type word goes to its group in the
+// provisional list of the particle's sorted position, SPH_NBRS_ROW consecutive
+// words per position (group A from the front, B from the back).  The parts
+// are apart because they diverge differently: the lanes of a warp have about
+// as many candidates per cell, so the first runs in step, and about as many
+// neighbours in all but not per cell, so the second is balanced only over the
+// whole stencil.  Warp instructions for 229,535 particles off the lattice: 83 M;
+// with the bits visited cell by cell 149 M; with the store path inside the
+// test loop 112 M and 21 of 32 lanes active, and a resolve pass after it.  All
+// loops run while any lane needs them: without that the lanes drift apart and
+// the scan ran five times slower.  4.45 M particles: 4.28 + 1.77 ms with the
+// resolve pass, 2.62 ms now, of which the pair-record pass takes back 0.46 for
+// reading the provisional lists.  Bound by latency: 45% of issue slots at 7
+// blocks per SM (6: 2.71 ms; 8, with spills: 3.06).
+// The pair-record pass (k_pairw) runs one thread per particle in the
+// held order, reads its provisional list and writes list and records row by
+// row.
+
+// a pair of FP32 values and the packed operations on it (one instruction for
+// two candidates)
+__device__ __forceinline__ unsigned long long f32x2(float a, float b)
 {
-    const int q = IDX, N = d.p.N;
-    if (q >= N || *d.s.err) return;
-    int np = 0;   // provisional entries
-    const int pid = d.s.pid_sorted[q];
-    if (d.s.type[pid] != 7) {
-        constexpr int nst = (ND == 2) ? 9 : 27;
-        constexpr float U = 5.9604645e-8f;     // 2^-24
-        const float4* xsf = reinterpret_cast<const float4*>(d.s.xsf);
-        const int nc = (int)d.s.key_out[q];
-        const float4 fi = xsf[q];              // the particle's own FP32 record
-        const float fz = (ND == 3) ? fi.z : 0.f;
-        float Fi = fmaxf(fabsf(fi.x), fabsf(fi.y));
-        if (ND == 3) Fi = fmaxf(Fi, fabsf(fz));
-        if (!(fi.w > 64.f * U * Fi)) {
-            np = -1;
-        } else {
-            const Prefilter P = make_prefilter<ND>(fi.x, fi.y, fz, fi.w, 2.2f * U * Fi, 32.f * U);
-            const CellGrid g = cell_grid(d, pid);
-            int* row = d.s.nbrs + q;
-            for (int nj = 0; nj < nst; nj++) {
-                const int nl = cell_link<ND>(g, nc, nj);
-                if (nl <= 0) continue;
-                const int start = d.s.cstart[nl], end = d.s.cend[nl];
-                for (int c = start; c <= end; c++) {
-                    const float4 fc = xsf[c];
-                    const int w = d.s.pts[c];
-                    const int v = nnps_prefilter<ND>(P, fc);
-                    if (v != 0) {
-                        if (np < SPH_NB_CAP) row[(size_t)np * N] = (v > 0) ? w : ~w;
-                        np++;
-                    }
-                }
-            }
-        }
-    }
-    d.s.nps[q] = np;
+    return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
-// The resolve pass of the search (see k_nnps), one thread per particle.
 template <int ND>
-__global__ void __launch_bounds__(128, SPH_MINB) k_nnps_resolve(Dev d)
+__global__ void __launch_bounds__(128, SPH_MINB_NNPS) k_nnps(Dev d)
 {
-    const int i = IDX, N = d.p.N;
-    if (i >= N || *d.s.err) return;
-    const int ti = d.s.type[i];
-    ListOut out(d, ti);
-    if (ti != 7) {
-        const int q0 = d.s.sortpos[i];
-        const int np = d.s.nps[q0];
-        const Pos pi = load_pos(d.s.xh, i);
-        if (np < 0 || np > SPH_NB_CAP) {
-            constexpr float U = 5.9604645e-8f;     // 2^-24
-            const float4 fi = reinterpret_cast<const float4*>(d.s.xsf)[q0];
-            const float fz = (ND == 3) ? fi.z : 0.f;
-            float Fi = fmaxf(fabsf(fi.x), fabsf(fi.y));
-            if (ND == 3) Fi = fmaxf(Fi, fabsf(fz));
-            const Prefilter P = make_prefilter<ND>(fi.x, fi.y, fz, fi.w, 2.2f * U * Fi, 32.f * U);
-            nnps_direct<ND>(d, i, d.s.cell[i], pi, np >= 0, P, out);
-        } else {
-            const double xi[3] = {pi.x, pi.y, pi.z};
-            const int* row = d.s.nbrs + q0;
-            // provisional entries two slots ahead
-            int v1 = (np > 0) ? row[0] : 0, v2 = (np > 1) ? row[N] : 0;
-            for (int s = 0; s < np; s++) {
-                const int v = v1;
-                v1 = v2;
-                if (s + 2 < np) v2 = row[(size_t)(s + 2) * N];
-                const int w = (v < 0) ? ~v : v, j = w >> 3;
-                const bool in = (v >= 0) || nnps_in_fp64<ND>(xi, pi.h, load_pos(d.s.xh, j));
-                if (in && j != i) out.add(d, i, w);
-            }
-        }
+    constexpr int nst = (ND == 2) ? 9 : 27;
+    constexpr float U = 5.9604645e-8f;     // 2^-24
+    constexpr unsigned ALL = 0xffffffffu;
+    // per stencil cell and thread: the first position looked at (a multiple
+    // of 4) and the bits of the 32 from it on
+    __shared__ int base[nst][128];
+    __shared__ unsigned bits[nst][128];
+    const int q = IDX, N = d.p.N, me = threadIdx.x;
+    if (*d.s.err) return;
+    int cnt = 0, na = 0, nb = 0;
+    const int pid = (q < N) ? d.s.pid_sorted[q] : 0;
+    const int ti = (q < N) ? d.s.type[pid] : 7;
+    const bool live = ti != 7;
+    const float4* xsf = reinterpret_cast<const float4*>(d.s.xsf);
+    const CellGrid g = cell_grid(d, pid);
+    const Pos own = load_pos(d.s.xs, live ? q : 0);
+    const float fx = (float)(own.x - g.xmin), fy = (float)(own.y - g.ymin);
+    const float fz = (ND == 3) ? (float)(own.z - g.zmin) : 0.f, fh = (float)own.h;
+    float Fi = fmaxf(fabsf(fx), fabsf(fy));
+    if (ND == 3) Fi = fmaxf(Fi, fabsf(fz));
+    float lo, hi;
+    prefilter_bounds<ND>(fh, 2.2f * U * Fi, &lo, &hi);
+    if (!(fh > 64.f * U * Fi && fh == (float)d.p.dr)) {
+        // every candidate to the FP64 test
+        lo = __int_as_float(0xff800000);
+        hi = __int_as_float(0x7f800000);
     }
-    out.store(d, i);
+    const Groups grp = list_groups(d, ti);
+    int* row = d.s.nbrs + (size_t)min(q, N - 1) * SPH_NBRS_ROW;
+
+    // one set bit: the candidate at position c, its record f
+    auto visit = [&](int c, const float4& f) {
+        if (c == q) return;                    // the particle itself
+        float t = fx - f.x;
+        float d2f = t * t;
+        t = fy - f.y;
+        d2f = __fmaf_rn(t, t, d2f);
+        if (ND == 3) {
+            t = fz - f.z;
+            d2f = __fmaf_rn(t, t, d2f);
+        }
+        if (!(d2f < lo)) {
+            const Pos pi = load_pos(d.s.xs, q);
+            const double xi[3] = {pi.x, pi.y, pi.z};
+            if (!nnps_in_fp64<ND>(xi, pi.h, load_pos(d.s.xs, c))) return;
+        }
+        const int w = __float_as_int(f.w);
+        cnt++;
+        if (cnt > SPH_NB_CAP) raise_err(d.s.err, SPH_ERR_NEIGH);
+        else if ((grp.a >> (w & 7)) & 1u) row[na++] = w;
+        else if ((grp.b >> (w & 7)) & 1u) row[SPH_NBRS_ROW - 1 - nb++] = w;
+    };
+    // the set bits of the stencil cells [n0, n1), in order, the records of two
+    // candidates ahead on their way
+    auto flush = [&](int n0, int n1) {
+        int nj = n0, c0 = 0;
+        unsigned m = 0u;
+        auto pop = [&]() {
+            while (m == 0u && nj < n1) {
+                m = bits[nj][me];
+                c0 = base[nj][me];
+                nj++;
+            }
+            if (m == 0u) return -1;
+            const int k = __ffs(m) - 1;
+            m &= m - 1;
+            return c0 + k;
+        };
+        int c1 = pop();
+        float4 f1 = xsf[max(c1, 0)];
+        int c2 = pop();
+        float4 f2 = xsf[max(c2, 0)];
+        while (__any_sync(ALL, c1 >= 0)) {
+            const int c3 = pop();
+            const float4 f3 = xsf[max(c3, 0)];
+            if (c1 >= 0) visit(c1, f1);
+            c1 = c2; f1 = f2;
+            c2 = c3; f2 = f3;
+        }
+    };
+
+    const size_t NP = (size_t)SPH_XSP_STRIDE(N);
+    const unsigned long long nx = f32x2(-fx, -fx), ny = f32x2(-fy, -fy), nz = f32x2(-fz, -fz);
+    const unsigned long long hi2 = f32x2(hi, hi), minus = f32x2(-1.f, -1.f);
+    // bits of the positions [p, p + 32), p a multiple of 4, n of them looked
+    // at: the sign of hi - d2 is 1 for a candidate outside (NaN: 0)
+    auto test = [&](int p, int n) {
+        const float* px = d.s.xsp + p;
+        unsigned m = 0u;
+        for (int k = 0; k < n; k += 4, px += 4) {
+            const float4 X = *reinterpret_cast<const float4*>(px), Y = *reinterpret_cast<const float4*>(px + NP);
+            unsigned long long a = add2(f32x2(X.x, X.y), nx), b = add2(f32x2(X.z, X.w), nx);
+            unsigned long long da = mul2(a, a), db = mul2(b, b);
+            a = add2(f32x2(Y.x, Y.y), ny); b = add2(f32x2(Y.z, Y.w), ny);
+            da = fma2(a, a, da); db = fma2(b, b, db);
+            if (ND == 3) {
+                const float4 Z = *reinterpret_cast<const float4*>(px + 2 * NP);
+                a = add2(f32x2(Z.x, Z.y), nz); b = add2(f32x2(Z.z, Z.w), nz);
+                da = fma2(a, a, da); db = fma2(b, b, db);
+            }
+            da = fma2(da, minus, hi2); db = fma2(db, minus, hi2);
+            m = __funnelshift_l((unsigned)da, m, 1);
+            m = __funnelshift_l((unsigned)(da >> 32), m, 1);
+            m = __funnelshift_l((unsigned)db, m, 1);
+            m = __funnelshift_l((unsigned)(db >> 32), m, 1);
+        }
+        return ~__brev(m << (32 - ((n + 3) & ~3)));
+    };
+
+    const int lc = live ? (int)d.s.key_out[q] - g.base : 0;
+    const int s1 = (ND == 2) ? 1 : g.czm, s2 = (ND == 2) ? g.cym : g.cxm * g.czm;
+    // stencil cell nj in cell_link's order: 2-D ky, kx; 3-D kz, kx, ky (the
+    // last fastest); its range of positions, loaded one cell ahead
+    auto range = [&](int nj, int& start, int& end) {
+        const int v = lc + ((ND == 2) ? (nj % 3 - 1) * s2 + (nj / 3 - 1) * s1
+                                      : (nj % 3 - 1) * s2 + ((nj / 3) % 3 - 1) * s1 + nj / 9 - 1);
+        start = 0;
+        end = -1;
+        if (live && v > 0 && v <= g.ctotal) {
+            start = d.s.cstart[v + g.base];
+            end = d.s.cend[v + g.base];
+        }
+    };
+    int done = 0, nexts, nexte;                // cells whose bits were visited
+    range(0, nexts, nexte);
+    for (int nj = 0; nj < nst; nj++) {
+        int start = nexts, len = nexte - nexts + 1;
+        if (nj + 1 < nst) range(nj + 1, nexts, nexte);
+        if (len <= 0) start = len = 0;
+        const int p = start & ~3, n = len ? start - p + len : 0;
+        const int longest = __reduce_max_sync(ALL, n);
+        unsigned m = 0u;
+        if (longest == 0) {
+        } else if (longest <= 32) {
+            m = test(p, longest);
+            m &= n ? (0xffffffffu >> (32 - n)) & (0xffffffffu << (start - p)) : 0u;
+        } else {
+            // a cell of more positions than bits: what is pending, then this
+            // cell 32 positions at a time
+            flush(done, nj);
+            for (int c = 0; c < longest; c += 32) {
+                const int left = n - c, pb = (left > 0) ? p + c : 0;
+                m = test(pb, min(32, longest - c));
+                if (left <= 0) m = 0u;
+                else if (left < 32) m &= (1u << left) - 1u;
+                if (c == 0) m &= 0xffffffffu << (start - p);
+                while (__any_sync(ALL, m != 0u))
+                    if (m) {
+                        const int k = __ffs(m) - 1;
+                        m &= m - 1;
+                        visit(pb + k, xsf[pb + k]);
+                    }
+            }
+            done = nj + 1;
+        }
+        bits[nj][me] = m;
+        base[nj][me] = p;
+    }
+    flush(done, nst);
+    if (q < N) {
+        d.s.nps[q] = na | (nb << 8);
+        d.s.nnb[pid] = cnt;
+    }
 }
 
 // The pair records of every list row, as partisearching stores wij with the
@@ -604,49 +637,54 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_nnps_resolve(Dev d)
 // in FP32 from the FP64 position differences in the bulk form; for group B
 // the kernel value alone.  One thread per particle walks its list, so for
 // each row a warp writes consecutive values.
+//
+// The rows come from the provisional list of the particle's sorted position
+// (src: four words a load, in group B backwards from the end of its row).
 template <int ND, typename R, bool GRAD>
-__device__ __forceinline__ void pairw_rows(const Dev& d, const PairI<R>& I, R rra, int i, int n, int row0, int dir)
+__device__ __forceinline__ void pairw_rows(const Dev& d, const PairI<R>& I, R rra, int i, int n, const int4* src,
+                                           int row0, int dir, unsigned long long wall[2])
 {
     const ptrdiff_t step = dir * (ptrdiff_t)d.p.N;
     size_t off = (size_t)row0 * d.p.N + i;
-    const int* p = d.s.nbr + off;
-    if constexpr (sizeof(R) == 8) {
+    int4 v = (n > 0) ? *src : make_int4(0, 0, 0, 0);
+    for (int s = 0; s < n; s += 4) {
+        const int4 now = v;
+        src += dir;
+        if (s + 4 < n) v = *src;
+        const int w4[4] = {dir > 0 ? now.x : now.w, dir > 0 ? now.y : now.z, dir > 0 ? now.z : now.y,
+                           dir > 0 ? now.w : now.x};
         // two rows at a time: their chains of dependent FP64 operations
-        // interleave; the next two rows' words are loaded ahead
-        int j0 = (n > 0) ? p[0] >> 3 : i, j1 = (n > 1) ? p[step] >> 3 : i;
-        for (int s = 0; s < n; s += 2) {
-            const Pos pa = load_pos(d.s.xh, j0), pb = load_pos(d.s.xh, j1);
-            p += 2 * step;
-            if (s + 2 < n) j0 = p[0] >> 3;
-            j1 = (s + 3 < n) ? p[step] >> 3 : j0;
-            R wa[4], wb[4];
-            pair_w64<ND, GRAD>(d, I, rra, pa, wa);
-            pair_w64<ND, GRAD>(d, I, rra, pb, wb);
-            if (GRAD) store_g<ND, R>(d, off, wa);
-            store_v<R>(d, off, wa[3]);
+        // interleave
+#pragma unroll
+        for (int h = 0; h < 4; h += 2) {
+            if (s + h >= n) break;
+            const bool two = s + h + 1 < n;
+            const int wa = w4[h], wb = two ? w4[h + 1] : wa;
+            const Pos pa = load_pos(d.s.xh, wa >> 3), pb = load_pos(d.s.xh, wb >> 3);
+            R ra[4], rb[4];
+            if constexpr (sizeof(R) == 8) {
+                pair_w64<ND, GRAD>(d, I, rra, pa, ra);
+                pair_w64<ND, GRAD>(d, I, rra, pb, rb);
+            } else {
+                pair_w_raw<ND, R>(d, I, rra, pa, ra);
+                pair_w_raw<ND, R>(d, I, rra, pb, rb);
+            }
+            d.s.nbr[off] = wa;
+            if (GRAD) store_g<ND, R>(d, off, ra);
+            store_v<R>(d, off, ra[3]);
             off += step;
-            if (s + 1 < n) {
-                if (GRAD) store_g<ND, R>(d, off, wb);
-                store_v<R>(d, off, wb[3]);
+            if (two) {
+                d.s.nbr[off] = wb;
+                if (GRAD) store_g<ND, R>(d, off, rb);
+                store_v<R>(d, off, rb[3]);
             }
             off += step;
+            if (GRAD) {
+                const int r = s + h;
+                if ((wa & 7) == 0) wall[r >> 6] |= 1ull << (r & 63);
+                if (two && (wb & 7) == 0) wall[(r + 1) >> 6] |= 1ull << ((r + 1) & 63);
+            }
         }
-        return;
-    }
-    // the next row's index and position are loaded one row ahead
-    Pos pn = load_pos(d.s.xh, (n > 0) ? *p >> 3 : i);
-    p += step;
-    int jn = (n > 1) ? *p >> 3 : 0;
-    for (int s = 0; s < n; s++) {
-        const Pos pj = pn;
-        p += step;
-        if (s + 1 < n) pn = load_pos(d.s.xh, jn);
-        if (s + 2 < n) jn = *p >> 3;
-        R w[4];
-        pair_w_raw<ND, R>(d, I, rra, pj, w);
-        if (GRAD) store_g<ND, R>(d, off, w);
-        store_v<R>(d, off, w[3]);
-        off += step;
     }
 }
 
@@ -655,9 +693,14 @@ __device__ __forceinline__ void pairw_particle(const Dev& d, int i)
 {
     const PairI<R> I = pair_i<ND, R>(d, i);
     const R rra = R(1.0) / I.h;     // RN(1 / h_i), the reciprocal of ra when h_j = h_i
-    const int n = d.s.nab[i];
-    pairw_rows<ND, R, true>(d, I, rra, i, n & 0xff, 0, 1);
-    pairw_rows<ND, R, false>(d, I, rra, i, n >> 8, SPH_NB_CAP - 1, -1);
+    const int q0 = d.s.sortpos[i], n = d.s.nps[q0];
+    const int4* src = reinterpret_cast<const int4*>(d.s.nbrs) + (size_t)q0 * (SPH_NBRS_ROW / 4);
+    unsigned long long wall[2] = {0ull, 0ull};
+    pairw_rows<ND, R, true>(d, I, rra, i, n & 0xff, src, 0, 1, wall);
+    pairw_rows<ND, R, false>(d, I, rra, i, n >> 8, src + SPH_NBRS_ROW / 4 - 1, SPH_NB_CAP - 1, -1, wall);
+    d.s.nab[i] = n;
+    d.s.nbm[i] = wall[0];
+    d.s.nbm[(size_t)d.p.N + i] = wall[1];
 }
 
 template <int ND>
@@ -3158,12 +3201,11 @@ extern "C" int sphk_enqueue_nnps_parts(const Dev* dp, void* sort_tmp, size_t sor
         REC(4);
         LAUNCH_ND(k_nnps, nblk(N, tbk(d, TP_NNPS)), tbk(d, TP_NNPS), d); n++;
         REC(5);
-        LAUNCH_ND(k_nnps_resolve, nblk(N, tbk(d, TP_RESOLVE)), tbk(d, TP_RESOLVE), d); n++;
         REC(6);
+        LAUNCH_ND(k_pairw, nblk(N, tbk(d, TP_PAIRW)), tbk(d, TP_PAIRW), d); n++;
 #if SPHGPU_CHECK
         k_check_lists<<<nblk(N, 128), 128, 0, st>>>(d); n++;
 #endif
-        LAUNCH_ND(k_pairw, nblk(N, tbk(d, TP_PAIRW)), tbk(d, TP_PAIRW), d); n++;
     }
     if (parts & 4) {
         REC(7);
