@@ -72,9 +72,9 @@ PASS_BYTES_2D = {
 STEP_BYTES_3D = 1870.0
 PASS_KERNELS = {
     "key": ("k_cellkey",),
-    "radix sort": ("radix_sort",),
+    "radix sort": ("k_cellscan", "k_cellplace"),
     "reorder": ("reorder",),
-    "cell ranges": ("k_cellreset", "k_cellrange"),
+    "cell ranges": ("k_cellrange",),
     "porosity + continuity": ("k_density",),
     "Shepard + EOS": ("k_shepard_eos",),
     "strain + stress + free surface + eigen": ("k_strain", "k_regu_eps", "k_saturation", "k_stress",

@@ -232,8 +232,8 @@ int sphgpu_step(sphgpu_ctx* ctx, int nsteps);
  * Step l in the reference's method granularity, for the C++ shim classes that
  * keep SPH_Calculation's own loop (CPP_1-SPHLoops.cpp:523-753) as the caller:
  *   sphgpu_parttocell      clNNPS_Fun::parttocell (CPP_3-NNPS.cpp:175-263):
- *                          cell keys, the radix sort in Binary_Sort's order and
- *                          the cell ranges; returns 0 or 3
+ *                          cell keys, Binary_Sort's order and the cell
+ *                          ranges; returns 0 or 3
  *   sphgpu_partisearching  clNNPS_Fun::partisearching (CPP_3-NNPS.cpp:265-374):
  *                          the neighbour lists and their kernel values; runs
  *                          parttocell first if the step has not; returns 0 or 5
@@ -446,7 +446,7 @@ void*  sphgpu_stream(sphgpu_ctx* ctx);
  * directly on the context's stream with a CUDA event between consecutive
  * stages, and adds each stage's duration (ms, summed over the steps) to
  * stage_ms[0 .. sphgpu_stage_count()-1].  Stage k is named by
- * sphgpu_stage_name(k) (the kernel names, plus "radix_sort").
+ * sphgpu_stage_name(k) (the kernel names).
  */
 int         sphgpu_stage_count(void);
 const char* sphgpu_stage_name(int k);

@@ -25,11 +25,9 @@
 #include "../../include/sphgpu.h"
 #include "sph_device.cuh"
 
-extern "C" size_t sphk_sort_temp_bytes(int N, int end_bit);
-extern "C" int sphk_enqueue_nnps(const Dev* d, void* sort_tmp, size_t sort_bytes, int end_bit, cudaStream_t st,
-                                 cudaEvent_t* ev);
-extern "C" int sphk_enqueue_nnps_parts(const Dev* d, void* sort_tmp, size_t sort_bytes, int end_bit,
-                                       cudaStream_t st, cudaEvent_t* ev, int parts);
+extern "C" size_t sphk_cell_slots(int ctotal);
+extern "C" int sphk_enqueue_nnps(const Dev* d, cudaStream_t st, cudaEvent_t* ev);
+extern "C" int sphk_enqueue_nnps_parts(const Dev* d, cudaStream_t st, cudaEvent_t* ev, int parts);
 extern "C" int sphk_enqueue_physics(const Dev* d, cudaStream_t st, cudaEvent_t* ev, int regu);
 extern "C" int sphk_enqueue_physics_bulk32(const Dev* d, cudaStream_t st, cudaEvent_t* ev, int regu);
 extern "C" const char* const sphk_stage_names[];
@@ -137,9 +135,6 @@ struct sphgpu_ctx {
     Dev d[2];              // parity variants: d[p] reads buffers "cur" of parity p
     int parity = 0;
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
-    void* sort_tmp = nullptr;
-    size_t sort_bytes = 0;
-    int end_bit = 1;
     std::vector<void*> allocs;
     // filled whole by whoever sizes them, so left uninitialised until then
     std::vector<int, UninitAlloc<int>> h_type, h_matype;
@@ -328,13 +323,6 @@ int alloc_optional(sphgpu_ctx* c, const sphgpu_params* P)
     return r;
 }
 
-int end_bit_for(int m)
-{
-    int b = 1;
-    while (b < 32 && (1u << b) <= (unsigned)m) b++;
-    return b;
-}
-
 // the physics stages of one step in the context's precision form
 int enqueue_physics(const sphgpu_ctx* c, const Dev* d, cudaEvent_t* ev)
 {
@@ -350,7 +338,7 @@ int build_graphs(sphgpu_ctx* c)
         if (c->exec[p]) { cudaGraphExecDestroy(c->exec[p]); c->exec[p] = nullptr; }
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-        int n = sphk_enqueue_nnps(&c->d[p], c->sort_tmp, c->sort_bytes, c->end_bit, c->st, nullptr);
+        int n = sphk_enqueue_nnps(&c->d[p], c->st, nullptr);
         n += enqueue_physics(c, &c->d[p], nullptr);
         cudaError_t e = cudaStreamEndCapture(c->st, &g);
         if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
@@ -916,7 +904,8 @@ sphgpu_ctx* sphgpu_create(const sphgpu_params* P, int device)
     if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess) return fail(SPHGPU_E_CUDA);
     cudaEventCreate(&c->ev0);
     cudaEventCreate(&c->ev1);
-    const int N = c->N, M = P->ctotal + 4;
+    const int N = c->N;
+    const size_t M = sphk_cell_slots(P->ctotal);   // cells 0 .. ctotal, whole blocks of the scan
     Dev& d = c->d[0];
     fill_dev_params(d.p, P);
     DevState& s = d.s;
@@ -950,8 +939,9 @@ sphgpu_ctx* sphgpu_create(const sphgpu_params* P, int device)
     r |= dalloc(c, &s.vsig, N); r |= dalloc(c, &s.veps, N); r |= dalloc(c, &s.divq, N); r |= dalloc(c, &s.divr, N);
     r |= dalloc(c, &s.meps, N);
     r |= dalloc(c, &s.i2o, N); r |= dalloc(c, &s.o2i, N);
-    r |= dalloc(c, &s.cell, N); r |= dalloc(c, &s.key_in, N); r |= dalloc(c, &s.key_out, N);
-    r |= dalloc(c, &s.val_in, N); r |= dalloc(c, &s.pid_sorted, N);
+    r |= dalloc(c, &s.cell, N); r |= dalloc(c, &s.ckey, N); r |= dalloc(c, &s.pid_sorted, N);
+    r |= dalloc(c, &s.placed, N); r |= dalloc(c, &s.ccount, sphk_cell_slots(P->ctotal)); r |= dalloc(c, &s.cofs, M);
+    r |= dalloc(c, &s.csum, sphk_cell_slots(P->ctotal) / SPH_SCAN_CELLS);
     r |= dalloc(c, &s.cstart, M); r |= dalloc(c, &s.cend, M);
     r |= dalloc(c, &s.nnb, N); r |= dalloc(c, &s.nbr, (size_t)SPH_NB_CAP * N);
     r |= dalloc(c, &s.nps, N); r |= dalloc(c, &s.sortpos, N);
@@ -973,10 +963,6 @@ sphgpu_ctx* sphgpu_create(const sphgpu_params* P, int device)
         return fail(SPHGPU_E_CUDA);
     k_order_identity<<<(N + 255) / 256, 256, 0, c->st>>>(s.i2o, s.o2i, N);
     if (cudaPeekAtLastError() != cudaSuccess) return fail(SPHGPU_E_CUDA);
-    c->end_bit = end_bit_for(P->ctotal);
-    c->sort_bytes = sphk_sort_temp_bytes(N, c->end_bit);
-    if (cudaMalloc(&c->sort_tmp, c->sort_bytes + 256) != cudaSuccess) return fail(SPHGPU_E_CUDA);
-    c->allocs.push_back(c->sort_tmp);
     // the staging buffers of the record transfers, sized for Particle and
     // material records, allocated with the rest of the state
     if (ensure_rec_staging(c, (size_t)kRecChunk * std::max({(size_t)kParticleBytes, sizeof(sphgpu_fluid),
@@ -1491,7 +1477,7 @@ int run_parts(sphgpu_ctx* c, int upto)
     if (c->part_done < 1 && upto >= 1) parts |= 1;
     if (c->part_done < 2 && upto >= 2) parts |= 2;
     if (upto >= 3) parts |= 4;
-    if (parts) sphk_enqueue_nnps_parts(d, c->sort_tmp, c->sort_bytes, c->end_bit, c->st, nullptr, parts);
+    if (parts) sphk_enqueue_nnps_parts(d, c->st, nullptr, parts);
     if (upto >= 3) {
         if (!c->regu && c->l_host % c->P.step_regu == 0) { c->regu = true; invalidate_graphs(c); }
         enqueue_physics(c, d, nullptr);
@@ -2276,7 +2262,7 @@ int sphgpu_nnps(sphgpu_ctx* c, int* ninflu, int* influ)
     // the lists whole, in list order
     Dev whole = c->d[c->parity];
     whole.p.split = 0;
-    sphk_enqueue_nnps_parts(&whole, c->sort_tmp, c->sort_bytes, c->end_bit, c->st, nullptr, 3);
+    sphk_enqueue_nnps_parts(&whole, c->st, nullptr, 3);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->st));
     int err = 0;
@@ -2296,7 +2282,7 @@ int sphgpu_nnps(sphgpu_ctx* c, int* ninflu, int* influ)
     }
     if (c->part_done >= 2 && err == 0) {
         // the lists of the step that sphgpu_update will complete
-        sphk_enqueue_nnps_parts(&c->d[c->parity], c->sort_tmp, c->sort_bytes, c->end_bit, c->st, nullptr, 2);
+        sphk_enqueue_nnps_parts(&c->d[c->parity], c->st, nullptr, 2);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(c->st));
     }
@@ -2345,7 +2331,7 @@ int sphgpu_step_profiled(sphgpu_ctx* c, int nsteps, double* stage_ms)
             cudaEventElapsedTime(&ms, c->ev0, c->ev1);
             c->reorder_ms += ms;
         }
-        sphk_enqueue_nnps(d, c->sort_tmp, c->sort_bytes, c->end_bit, c->st, ev);
+        sphk_enqueue_nnps(d, c->st, ev);
         enqueue_physics(c, d, ev);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(c->st));

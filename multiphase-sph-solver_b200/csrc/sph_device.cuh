@@ -40,6 +40,7 @@
 // values per plane of the search's position planes: whole lines, and room to
 // read up to 35 positions past the last
 #define SPH_XSP_STRIDE(N) (((N) + 36 + 63) / 64 * 64)
+#define SPH_SCAN_CELLS 1024    // cells per block of the cell scan: 4 per thread
 #define SPH_ERR_CELL 3         // parttocell, CPP_3-NNPS.cpp:247-257
 #define SPH_ERR_NEIGH 5        // partisearching, CPP_3-NNPS.cpp:313-319
 #define SPHK_NSTAGES 21        // entries of sphk_stage_names (one event bracket each)
@@ -203,8 +204,10 @@ struct DevState {
     int *i2o, *o2i;
     // NNPS
     int *cell;                 // cell id per particle
-    uint32_t *key_in, *key_out;
-    int *val_in, *pid_sorted;
+    int *ccount;               // particles per cell, zero between steps
+    int *csum, *cofs;          // particles per run of SPH_SCAN_CELLS cells; per cell, its first position
+    int2 *placed;              // per position of a cell in placing order: particle, its caller's index
+    int *ckey, *pid_sorted;    // per sorted position: cell, particle
     int *cstart, *cend;        // [ctotal + 4]
     int *nnb;                  // neighbour count (may exceed the cap: error 5)
     // the neighbour search by cell-sorted position q: the scan's group sizes

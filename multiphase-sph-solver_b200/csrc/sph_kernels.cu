@@ -6,9 +6,9 @@
 // dependency chain:
 //
 //   k_cellkey      parttocell: cell key per particle            (CPP_3-NNPS.cpp:175-257)
-//   radix sort     Binary_Sort's order: cell ascending, index descending
-//   k_cellreset    cell_info reset                              (CPP_3-NNPS.cpp:196-201)
-//   k_cellrange    cell_info start/end (:621-629) + the cell-sorted copy of positions
+//   k_cellscan     cell_info start/end                          (CPP_3-NNPS.cpp:196-201, :621-629)
+//   k_cellplace, k_cellrange  Binary_Sort's order (cell ascending, index descending) and the
+//                  cell-sorted copy of positions
 //   k_nnps         partisearching: stencil scan in cell-sorted order, FP32 prefilter,
 //                  FP64 decisions of the undecided candidates
 //   k_pairw        neighbour lists and pair records in the held order
@@ -228,13 +228,7 @@ __global__ void k_cellkey(Dev d)
     }
     c += g.base;
     d.s.cell[i] = c;
-    // placed by the particle's index in the caller's order, reversed: the
-    // stable radix sort then keeps equal keys in descending caller's index,
-    // the order Binary_Sort's merge produces, in whatever order the state is
-    // held
-    const int o = d.s.i2o[i];
-    d.s.key_in[N - 1 - o] = (uint32_t)c;
-    d.s.val_in[N - 1 - o] = i;
+    atomicAdd(&d.s.ccount[c], 1);
 }
 
 // rainpro (CPP_15-1-rain.cpp:43-85), at the top of the steps with
@@ -297,43 +291,110 @@ __global__ void __launch_bounds__(256) k_rain(Dev d)
     if (threadIdx.x == 0) *d.s.nrain = nrain - (end - k0 + 1);
 }
 
-__global__ void k_cellreset(Dev d)
+// Binary_Sort's order (cell ascending, index descending, CPP_3-NNPS.cpp:
+// 561-630) by counting: the particles per cell (k_cellkey), the cells' first
+// positions (k_cellsum, k_cellscan), each particle into its cell's positions in
+// any order (k_cellplace), and its rank among the cell's particles
+// (k_cellrange).  A cell holds a handful of particles, so the rank costs a few
+// broadcast loads, and the order does not depend on which particle was placed
+// first.  A radix sort of the keys moved every particle two or three times in
+// six launches; with it, the cells' reset and the ranges a step of 14,978
+// particles took 0.144 ms, with these passes 0.113 (0.21 and 0.23 ms of a step
+// of 4.45 M particles).
+
+// the particles in each run of SPH_SCAN_CELLS cells, four cells per thread
+__global__ void __launch_bounds__(SPH_SCAN_CELLS / 4) k_cellsum(Dev d)
 {
-    const int c = IDX;
-    if (c >= d.p.ctotal || *d.s.err) return;
-    if (d.p.ninst > 0) {
-        // each instance's own cell ctotal keeps its range, as in one system
-        int lo = 0, hi = d.p.ninst - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (d.s.inst[mid].cell_base <= c) lo = mid;
-            else hi = mid - 1;
-        }
-        if (c - d.s.inst[lo].cell_base == d.s.inst[lo].ctotal) return;
-    }
-    d.s.cstart[c] = 10000000;
-    d.s.cend[c] = -10000000;
+    if (*d.s.err) return;
+    typedef cub::BlockReduce<int, SPH_SCAN_CELLS / 4> Reduce;
+    __shared__ typename Reduce::TempStorage tmp;
+    const int4 v = reinterpret_cast<const int4*>(d.s.ccount)[(size_t)blockIdx.x * blockDim.x + threadIdx.x];
+    const int sum = Reduce(tmp).Sum(v.x + v.y + v.z + v.w);
+    if (threadIdx.x == 0) d.s.csum[blockIdx.x] = sum;
 }
 
-// cell_info start/end, and the positions in cell-sorted order.  Cell ctotal
-// is never reset by the reference (its reset loop stops at ctotal - 1), so its
-// range accumulates across steps.
+// cell_info (CPP_3-NNPS.cpp:196-201, 621-629): each cell's first position
+// (cofs) and its range.  Cell ctotal (each instance's own) is never reset by
+// the reference (its reset loop stops at ctotal - 1), so its range accumulates
+// across steps.  Short runs of cells and whole-vector stores: with 8,192 cells
+// per block and single stores the one or three blocks of a small grid took
+// 20 us on their stores alone.
+__global__ void __launch_bounds__(SPH_SCAN_CELLS / 4) k_cellscan(Dev d)
+{
+    if (*d.s.err) return;
+    typedef cub::BlockReduce<int, SPH_SCAN_CELLS / 4> Reduce;
+    typedef cub::BlockScan<int, SPH_SCAN_CELLS / 4> Scan;
+    __shared__ union { typename Reduce::TempStorage r; typename Scan::TempStorage s; } tmp;
+    __shared__ int before;
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int4 v = reinterpret_cast<const int4*>(d.s.ccount)[t];
+    int sum = 0;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += blockDim.x) sum += d.s.csum[b];
+    sum = Reduce(tmp.r).Sum(sum);
+    if (threadIdx.x == 0) before = sum;
+    __syncthreads();
+    int first;
+    Scan(tmp.s).ExclusiveSum(v.x + v.y + v.z + v.w, first);
+    first += before;
+    const int n[4] = {v.x, v.y, v.z, v.w};
+    int a[4], e[4];
+    for (int k = 0; k < 4; k++) {
+        a[k] = first;
+        e[k] = first + n[k] - 1;
+        first += n[k];
+    }
+    reinterpret_cast<int4*>(d.s.cofs)[t] = make_int4(a[0], a[1], a[2], a[3]);
+    for (int k = 0; k < 4; k++) {
+        const long long c = 4 * (long long)t + k;
+        bool keep = c == d.p.ctotal;
+        if (d.p.ninst > 0 && c < d.p.ctotal) {
+            int lo = 0, hi = d.p.ninst - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (d.s.inst[mid].cell_base <= c) lo = mid;
+                else hi = mid - 1;
+            }
+            keep = c - d.s.inst[lo].cell_base == d.s.inst[lo].ctotal;
+        }
+        if (keep) {
+            const int s0 = d.s.cstart[c], e0 = d.s.cend[c];
+            a[k] = n[k] > 0 ? min(s0, a[k]) : s0;
+            e[k] = n[k] > 0 ? max(e0, e[k]) : e0;
+        }
+    }
+    reinterpret_cast<int4*>(d.s.cstart)[t] = make_int4(a[0], a[1], a[2], a[3]);
+    reinterpret_cast<int4*>(d.s.cend)[t] = make_int4(e[0], e[1], e[2], e[3]);
+}
+
+// each particle into one of its cell's positions; the counts return to zero
+__global__ void k_cellplace(Dev d)
+{
+    const int i = IDX, N = d.p.N;
+    if (i >= N || *d.s.err) return;
+    const int c = d.s.cell[i];
+    const int q = d.s.cofs[c] + atomicSub(&d.s.ccount[c], 1) - 1;
+    d.s.placed[q] = make_int2(i, d.s.i2o[i]);
+}
+
+// each particle's sorted position: its cell's particles in descending caller's
+// index, the order Binary_Sort's merge produces, in whatever order the state
+// is held; and the positions in that order
 __global__ void k_cellrange(Dev d)
 {
-    const int q = IDX, N = d.p.N;
-    if (q >= N || *d.s.err) return;
-    const uint32_t c = d.s.key_out[q];
-    const bool first = (q == 0) || d.s.key_out[q - 1] != c;
-    const bool last = (q == N - 1) || d.s.key_out[q + 1] != c;
-    const int pid = d.s.pid_sorted[q];
-    const CellGrid g = cell_grid(d, pid);
-    if ((int)c - g.base == g.ctotal) {
-        if (first) atomicMin(&d.s.cstart[c], q);
-        if (last) atomicMax(&d.s.cend[c], q);
-    } else {
-        if (first) d.s.cstart[c] = q;
-        if (last) d.s.cend[c] = q;
+    const int p = IDX, N = d.p.N;
+    if (p >= N || *d.s.err) return;
+    const int2 me = d.s.placed[p];
+    const int pid = me.x, c = d.s.cell[pid], first = d.s.cofs[c];
+    // positions of the same cell on both sides of p
+    int q = first;
+    for (int r = first; r < N; r++) {
+        const int2 o = d.s.placed[r];
+        if (r > p && d.s.cell[o.x] != c) break;
+        q += o.y > me.y;
     }
+    const CellGrid g = cell_grid(d, pid);
+    d.s.pid_sorted[q] = pid;
+    d.s.ckey[q] = c;
     d.s.sortpos[pid] = q;
     const int t = d.s.type[pid];
     const int w = (pid << 3) | ((t >= 0 && t <= 4) ? t : 7);
@@ -576,7 +637,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_NNPS) k_nnps(Dev d)
         return ~__brev(m << (32 - ((n + 3) & ~3)));
     };
 
-    const int lc = live ? (int)d.s.key_out[q] - g.base : 0;
+    const int lc = live ? d.s.ckey[q] - g.base : 0;
     const int s1 = (ND == 2) ? 1 : g.czm, s2 = (ND == 2) ? g.cym : g.cxm * g.czm;
     // stencil cell nj in cell_link's order: 2-D ky, kx; 3-D kz, kx, ky (the
     // last fastest); its range of positions, loaded one cell ahead
@@ -3049,14 +3110,6 @@ static inline int tbk(const Dev& d, int pass)
 #define REC(k) do { if (ev) cudaEventRecord(ev[k], st); } while (0)
 
 #ifndef SPH_BULK32
-extern "C" size_t sphk_sort_temp_bytes(int N, int end_bit)
-{
-    size_t bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const uint32_t*)nullptr, (uint32_t*)nullptr,
-                                    (const int*)nullptr, (int*)nullptr, N, 0, end_bit);
-    return bytes;
-}
-
 // The order sphgpu_set_reorder re-sorts the particle state into: by type
 // and material (so that a warp's particles take the same branches of the
 // constitutive and momentum passes: co-located phases, such as the water
@@ -3126,7 +3179,7 @@ extern "C" int sphk_order_sort(const Dev* dp, void* tmp, size_t bytes, int end_b
 // before stage k and ev[SPHK_NSTAGES] after the last one (stages a run does
 // not need are recorded with no work between their events).
 extern "C" const char* const sphk_stage_names[] = {
-    "k_cellkey", "radix_sort", "k_cellreset", "k_cellrange", "k_nnps", "k_nnps_resolve", "k_pairw", "k_kgc",
+    "k_cellkey", "k_cellscan", "k_cellplace", "k_cellrange", "k_nnps", "k_nnps_resolve", "k_pairw", "k_kgc",
     "k_density", "k_shepard_eos", "k_strain", "k_regu_eps", "k_stress", "k_regu_sig", "k_stress_2",
     "k_art_rij", "k_accel_a", "k_accel_b", "k_xsph_update", "k_tm_boundary", "k_step_done"};
 static_assert(sizeof(sphk_stage_names) / sizeof(sphk_stage_names[0]) == SPHK_NSTAGES, "stage table");
@@ -3178,8 +3231,13 @@ __global__ void k_check_lists(Dev d)
 }
 #endif
 
-extern "C" int sphk_enqueue_nnps_parts(const Dev* dp, void* sort_tmp, size_t sort_bytes, int end_bit,
-                                       cudaStream_t st, cudaEvent_t* ev, int parts)
+// the cells the counts are kept for: whole blocks of the scan
+extern "C" size_t sphk_cell_slots(int ctotal)
+{
+    return ((size_t)ctotal + 1 + SPH_SCAN_CELLS - 1) / SPH_SCAN_CELLS * SPH_SCAN_CELLS;
+}
+
+extern "C" int sphk_enqueue_nnps_parts(const Dev* dp, cudaStream_t st, cudaEvent_t* ev, int parts)
 {
     const Dev& d = *dp;
     const int N = d.p.N;
@@ -3189,11 +3247,11 @@ extern "C" int sphk_enqueue_nnps_parts(const Dev* dp, void* sort_tmp, size_t sor
         if (d.p.flr) { LAUNCH_ND(k_rain, 1, 256, d); n++; }
         LAUNCH_ND(k_cellkey, nblk(N, 256), 256, d); n++;
         REC(1);
-        size_t bytes = sort_bytes;
-        cub::DeviceRadixSort::SortPairs(sort_tmp, bytes, d.s.key_in, d.s.key_out, d.s.val_in, d.s.pid_sorted,
-                                        N, 0, end_bit, st);
+        const unsigned blocks = (unsigned)(sphk_cell_slots(d.p.ctotal) / SPH_SCAN_CELLS);
+        if (blocks > 1) { k_cellsum<<<blocks, SPH_SCAN_CELLS / 4, 0, st>>>(d); n++; }
+        k_cellscan<<<blocks, SPH_SCAN_CELLS / 4, 0, st>>>(d); n++;
         REC(2);
-        k_cellreset<<<nblk(d.p.ctotal, 256), 256, 0, st>>>(d); n++;
+        k_cellplace<<<nblk(N, 256), 256, 0, st>>>(d); n++;
         REC(3);
         k_cellrange<<<nblk(N, 256), 256, 0, st>>>(d); n++;
     }
@@ -3214,10 +3272,9 @@ extern "C" int sphk_enqueue_nnps_parts(const Dev* dp, void* sort_tmp, size_t sor
     return n;
 }
 
-extern "C" int sphk_enqueue_nnps(const Dev* dp, void* sort_tmp, size_t sort_bytes, int end_bit, cudaStream_t st,
-                                 cudaEvent_t* ev)
+extern "C" int sphk_enqueue_nnps(const Dev* dp, cudaStream_t st, cudaEvent_t* ev)
 {
-    return sphk_enqueue_nnps_parts(dp, sort_tmp, sort_bytes, end_bit, st, ev, 7);
+    return sphk_enqueue_nnps_parts(dp, st, ev, 7);
 }
 #endif  // !SPH_BULK32
 

@@ -108,3 +108,17 @@ def test_far_from_the_grid_origin():
     xp[100:, 0] += 0.4e6 * dr
     xp[:, 2] = 0.0
     _search_equal(xp, 2, dr)
+
+
+@pytest.mark.parametrize("cells", ((31, 33), (32, 32), (64, 64), (41, 75), (200, 3), (3, 5)))
+def test_cell_counts_around_the_scan_blocks(cells):
+    """Grids whose number of cells is at, one past and far from a multiple of
+    what a block of the cell scan takes; particles at every corner."""
+    rng = np.random.default_rng(sum(cells))
+    dr = 0.1
+    ext = [2 * dr * (c - 2.5) - 4 * dr for c in cells]           # celllist_ini1 then gives these counts
+    xp = np.zeros((600, 3))
+    for k in range(2):
+        xp[:, k] = rng.random(600) * max(ext[k], 0.05)
+        xp[:4, k] = (0.0, max(ext[k], 0.05)) * 2 if k else (0.0, 0.0, max(ext[0], 0.05), max(ext[0], 0.05))
+    _search_equal(xp[:max(8, min(600, 4 * cells[0] * cells[1]))], 2, dr)
