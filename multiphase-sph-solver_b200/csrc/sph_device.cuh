@@ -150,9 +150,11 @@ struct DevState {
     double *vx_next;           // per particle (vx x, y, z before XSPH, mass): one 32-byte record
     double *vxp, *axp, *ax, *ux;
     double *rho, *rhop, *pre, *prep, *porosity, *poro_cop, *e;
-    double *rho_c;             // per particle (continuity density, mass): one 16-byte record for Shepard
+    double *rho_c;             // per particle (mass / continuity density, or in the bulk form that density;
+                               // mass): one 16-byte record for Shepard
     double *svr;               // per particle (vxp x, y, z, mass / rho) after Shepard: the strain loop's record
-    double *pmr;               // per particle (mass, rho, pre, 0) after Shepard: the pressure gathers' record
+    double *pmr;               // per particle (mass, rho, pre, RN(1 / rho)) after Shepard: the record of the
+                               // pressure gathers and XSPH
     double *dr4;               // per particle (rho, satu, porosity, soil: cop | fluid: f_dens) after the
                                // constitutive pass: the drag loop's record
     double *rrho;              // per particle (mass, porosity, rho, RN(1 / rho)) at the start of the step
@@ -488,6 +490,30 @@ __device__ __forceinline__ double div_rcp_fast(double x, double y, double yr, bo
     const int h = __double2hiint(r), l = __double2loint(r);
     bad |= (h & 0x7ff00000) == 0x7ff00000;
     return (((h << 1) | l) == 0) ? q : v;      // r = 0: q is exact, sign included
+}
+
+// v[k] / y for each k, y's correctly rounded reciprocal yr at hand (FP64); one
+// test for all of them in place of a division's slow path each.  The FP32
+// form divides.
+template <int K>
+__device__ __forceinline__ void quotients(double (&v)[K], double y, double yr)
+{
+    bool bad = false;
+    double q[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) q[k] = div_rcp_fast(v[k], y, yr, bad);
+    if (bad) {
+#pragma unroll
+        for (int k = 0; k < K; k++) q[k] = v[k] / y;
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = q[k];
+}
+template <int K>
+__device__ __forceinline__ void quotients(float (&v)[K], float y, double)
+{
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = v[k] / y;
 }
 
 // pair_w_raw in FP64 for h_j = h_i, the same operations in the same order with

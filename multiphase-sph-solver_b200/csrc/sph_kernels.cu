@@ -880,8 +880,12 @@ __global__ void __launch_bounds__(128, SPH_MINB_DENS) k_density(Dev d)
         else
             rnew = rhop + drhot * dt;
     }
-    // the continuity density with the mass, one record for the Shepard gathers
-    reinterpret_cast<double2*>(d.s.rho_c)[i] = make_double2(rnew, d.s.mass[i]);
+    // one record for the Shepard gathers: the mass with its quotient by the
+    // continuity density, which the reference forms per pair (the FP32-bulk
+    // form does too, from the density)
+    const double m = d.s.mass[i];
+    reinterpret_cast<double2*>(d.s.rho_c)[i] = make_double2(sizeof(real) == 8 ? m / rnew : rnew, m);
+    d.s.rho[i] = rnew;
 }
 
 // Shepard filter (:168-188) reading every neighbour's continuity density
@@ -904,10 +908,10 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_shepard_eos(Dev d)
         const double2 cm = reinterpret_cast<const double2*>(d.s.rho_c)[j];
         const real mj = (real)cm.y;
         sup.add(mj * w3);
-        sdown.add(mj / (real)cm.x * w3);
+        sdown.add((sizeof(real) == 8 ? (real)cm.x : mj / (real)cm.x) * w3);
     }
     const double up = sup.v(), down = sdown.v();
-    double r = reinterpret_cast<const double2*>(d.s.rho_c)[i].x;
+    double r = d.s.rho[i];         // the continuity density
     if (ti != 7 && fabs(down) > 1.0e-7) r = up / down;
     d.s.rho[i] = r;
     {
@@ -926,10 +930,9 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_shepard_eos(Dev d)
         double pr = prep * (pow7(r / d.s.rhop[i]) - 1.0);
         d.s.pre[i] = pr + prep;
     }
-    {
-        // the pressure gathers' record: mass, rho and pressure of this step
-        st_rec4(d.s.pmr, (size_t)i, d.s.mass[i], r, d.s.pre[i], 0.0);
-    }
+    // the pressure and XSPH gathers' record: mass, rho, pressure of this step,
+    // and RN(1 / rho) for their quotients by rho
+    st_rec4(d.s.pmr, (size_t)i, d.s.mass[i], r, d.s.pre[i], 1.0 / r);
 }
 
 // ---------------------------------------------------------------------------
@@ -1043,14 +1046,19 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRAIN) k_strain(Dev d)
         while (itg.next(j, tj, o)) {
             if (!(tj == 1 || tj == 3 || (tj == 2 && ti == 0))) continue;
             const real w3 = load_v<real>(d, o);
-            const NV pm = load_nv(d.s.pmr, j);      // (mass, rho, pre, -)
+            const NV pm = load_nv(d.s.pmr, j);      // (mass, rho, pre, 1 / rho)
             const real mj = (real)pm.vx, rj = (real)pm.vy;
             const real pj_ = (ti == 0 && tj == 2) ? real(0) : (real)pm.vz;
-            if (tj == 1) { su1.add(mj * pj_ * w3 / rj); sd1.add(mj * w3 / rj); }
-            if (tj == 3) { su2.add(mj * pj_ * w3 / rj); sd2.add(mj * w3 / rj); }
+            real v[2] = {mj * pj_ * w3, mj * w3};
+            quotients(v, rj, pm.m);
+            if (tj == 1) { su1.add(v[0]); sd1.add(v[1]); }
+            if (tj == 3) { su2.add(v[0]); sd2.add(v[1]); }
             if (ti == 0 && tj == 2) {
-                for (int k = 0; k < 6; k++) sus[k].add(mj * (real)d.s.sig[k * N + j] * w3 / rj);
-                sdsw.add(mj * w3 / rj);
+                real sv[6];
+                for (int k = 0; k < 6; k++) sv[k] = mj * (real)d.s.sig[k * N + j] * w3;
+                quotients(sv, rj, pm.m);
+                for (int k = 0; k < 6; k++) sus[k].add(sv[k]);
+                sdsw.add(v[1]);
             }
         }
         // gathered pressures (eos :122-176)
@@ -2146,11 +2154,15 @@ __global__ void __launch_bounds__(128, SPH_MINB_XSPH) k_xsph_update(Dev d)
             const real xishu = (tj == 0) ? xs_wall : xs_same;
             const real w3 = load_v<real>(d, o);
             const NV nj = load_nv(d.s.vx_next, j);
-            const real mj = (real)nj.m, rj = (real)d.s.rho[j];
+            const NV pm = load_nv(d.s.pmr, j);      // (mass, rho, pre, 1 / rho)
+            const real mj = (real)nj.m, rj = (real)pm.vy;
             const double vjs[3] = {nj.vx, nj.vy, nj.vz};
-            for (int k = 0; k < nd; k++)
-                stu[k].add(xishu * mj * (real)(vjs[k] - vm[k]) * w3 / rj);
-            sdown.add(mj * w3 / rj);
+            real v[nd + 1];
+            for (int k = 0; k < nd; k++) v[k] = xishu * mj * (real)(vjs[k] - vm[k]) * w3;
+            v[nd] = mj * w3;
+            quotients(v, rj, pm.m);
+            for (int k = 0; k < nd; k++) stu[k].add(v[k]);
+            sdown.add(v[nd]);
         }
         double tu[3];
         for (int k = 0; k < 3; k++) tu[k] = stu[k].v();
