@@ -272,6 +272,7 @@ void fill_dev_params(DevParams& p, const sphgpu_params* P)
     p.st_vpu = P->structure.vpu;
     p.ninst = 0;
     p.split = p.ss_coupled ? 0 : 1;
+    p.visc = 0;                        // set_visc
     for (int q = 0; q < TP_COUNT; q++) p.tb[q] = 128;
     p.flr = P->flr == 1 ? 1 : 0;
     p.rain_lp = 0; p.rain_vrain = 0.0; p.rain_press = 0.0;
@@ -665,6 +666,17 @@ void* field_ptr(sphgpu_ctx* c, const char* name)
     for (auto& t : tab)
         if (std::strcmp(t.n, name) == 0) return t.p;
     return nullptr;
+}
+
+// whether the strain pass takes the artificial-viscosity sums in the steps to
+// come: past inip no step damps again (its own loop also forms the damping and
+// vibration sums)
+void set_visc(sphgpu_ctx* c)
+{
+    const int want = c->precision == SPHGPU_PREC_FP64 && c->P.flv == 0 && c->l_host > c->P.inip;
+    if (c->d[0].p.visc == want) return;
+    for (int p = 0; p < 2; p++) c->d[p].p.visc = want;
+    invalidate_graphs(c);
 }
 
 // the first wall (index order) with matype > 2 in [a, b), or b
@@ -1480,6 +1492,7 @@ int run_parts(sphgpu_ctx* c, int upto)
     if (parts) sphk_enqueue_nnps_parts(d, c->st, nullptr, parts);
     if (upto >= 3) {
         if (!c->regu && c->l_host % c->P.step_regu == 0) { c->regu = true; invalidate_graphs(c); }
+        set_visc(c);
         enqueue_physics(c, d, nullptr);
     }
     CK(cudaGetLastError());
@@ -1633,6 +1646,7 @@ int sphgpu_step(sphgpu_ctx* c, int nsteps)
         for (long long l = c->l_host; l < (long long)c->l_host + nsteps; l++)
             if (l % c->P.step_regu == 0) { c->regu = true; invalidate_graphs(c); break; }
     cudaSetDevice(c->device);
+    set_visc(c);
     if (!c->exec[0] || !c->exec[1]) {
         r = build_graphs(c);
         if (r) return r;
@@ -2320,6 +2334,7 @@ int sphgpu_step_profiled(sphgpu_ctx* c, int nsteps, double* stage_ms)
     int err = 0;
     c->reorder_ms = 0.0;
     for (int s = 0; s < nsteps && err == 0; s++) {
+        set_visc(c);
         const Dev* d = &c->d[c->parity];
         if (c->reorder_every > 0 && c->since_sort >= c->reorder_every) {
             CK(cudaEventRecord(c->ev0, c->st));

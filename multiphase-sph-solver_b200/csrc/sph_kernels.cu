@@ -94,6 +94,9 @@ namespace SPH_NS {
 #ifndef SPH_MINB_STRAIN
 #define SPH_MINB_STRAIN 6
 #endif
+#ifndef SPH_MINB_STRAINV
+#define SPH_MINB_STRAINV 5
+#endif
 #ifndef SPH_MINB_ACCA
 #define SPH_MINB_ACCA 4
 #endif
@@ -944,8 +947,18 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_shepard_eos(Dev d)
 // color, prew, prea,
 // and the walls' gathered stress into sig_next (reads the soil stresses of
 // the previous step from sig).
-template <int ND>
-__global__ void __launch_bounds__(128, SPH_MINB_STRAIN) k_strain(Dev d)
+//
+// VISC = 1 also forms the artificial-viscosity sums of the momentum pass
+// (CPP_9-3-artificialvis.cpp:12-99): they run over the same rows and need only
+// positions, velocities and the densities Shepard left, so the pass that
+// streams these gradients anyway takes them, and k_accel_b's loop over the
+// own type is not run.  Chosen by the host for steps past inip without
+// vibration (that loop also forms the damping and vibration sums), in FP64.
+// 4.45 M particles: strain and momentum loops 1.70 + 4.15 -> 2.87 + 2.30 ms; 2-D
+// slopes (588,662) 0.092 + 0.168 -> 0.128 + 0.076.  At 5 blocks per SM in 3-D (4:
+// 3.25 ms, 6, spilling: 3.70), 6 in 2-D.
+template <int ND, int VISC>
+__global__ void __launch_bounds__(128, VISC && ND == 3 ? SPH_MINB_STRAINV : SPH_MINB_STRAIN) k_strain(Dev d)
 {
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
@@ -958,6 +971,15 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRAIN) k_strain(Dev d)
     const bool moving = (ti >= 1 && ti <= 4);
     Sum<real> sup[9], sdown[3];
     Sum<real> scolor;
+    // artificial viscosity coefficients of particle i
+    Sum<real> tav[3];
+    real ca = 0, aa = 0, bb = 0, ri = 0;
+    if (VISC && ti >= 1 && ti <= 3) {
+        ca = (ti == 2) ? (real)d.s.s_vpu[i] : (real)d.s.f_vpu[i];
+        aa = (real)d.p.av[ti - 1][0];
+        bb = (real)d.p.av[ti - 1][1];
+        ri = (real)d.s.rho[i];
+    }
     // the velocity-gradient and colour sums over i's own type and the walls,
     // for moving i
     RowIter it = rows_a(d, i);
@@ -998,8 +1020,30 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRAIN) k_strain(Dev d)
             sup[6].add(mr * dvx[2] * w[0]);
             sup[7].add(mr * dvx[2] * w[1]);
             sup[8].add(mr * dvx[2] * w[2]);
+            Pos pj = P;
+            if (VISC || solid) pj = load_pos(d.s.xh, j);
+            if (VISC && same) {
+                // (a structure particle's coefficients are zero, and so are its sums)
+                const double2 md = reinterpret_cast<const double2*>(d.s.pmr)[2 * (size_t)j];
+                const real mj = (real)md.x, rj = (real)md.y;
+                const double xi[3] = {P.x, P.y, P.z}, xj[3] = {pj.x, pj.y, pj.z};
+                real inprod = 0, dst = 0;
+                for (int k = 0; k < nd; k++) {
+                    const real dx = (real)(xi[k] - xj[k]);
+                    dst = dst + dx * dx;
+                    inprod = inprod + dvx[k] * dx;
+                }
+                const real hl = ((real)pj.h + (real)P.h) * real(0.5);
+                const real rou = (rj + ri) * real(0.5);
+                real paix = 0;
+                if (inprod < real(0)) {
+                    dst = sqrt(dst);
+                    const real myu = hl * inprod / (dst * dst + real(0.01) * hl * hl);
+                    paix = (-aa * ca * myu + bb * myu * myu) / rou;
+                }
+                for (int k = 0; k < nd; k++) tav[k].add(mj * paix * w[k]);
+            }
             if (solid) {
-                const Pos pj = load_pos(d.s.xh, j);
                 sdown[0].add(mr * (real)(P.x - pj.x) * w[0]);
                 sdown[1].add(mr * (real)(P.y - pj.y) * w[1]);
                 sdown[2].add(mr * (real)(P.z - pj.z) * w[2]);
@@ -1033,6 +1077,8 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRAIN) k_strain(Dev d)
             d.s.we[k * N + i] = we[k];
         }
         d.s.color[i] = scolor.v();
+        if (VISC)
+            for (int k = 0; k < 3; k++) d.s.accb[(size_t)k * N + i] = (double)tav[k].v();
     }
     // the pressure (and, for walls, stress) gathers of eos from the fluids
     // (and, for walls, the soil), in a loop of their own over those slots:
@@ -1913,8 +1959,8 @@ __global__ void __launch_bounds__(128, SPH_MINB_ACCB) k_accel_b_tail(Dev d)
     double tav[3], tin[3], tdm[3];
     for (int k = 0; k < 3; k++) {
         tav[k] = d.s.accb[(size_t)k * N + i];
-        tin[k] = d.s.accb[(size_t)(3 + k) * N + i];
-        tdm[k] = d.s.accb[(size_t)(6 + k) * N + i];
+        tin[k] = (d.p.fli >= 1) ? d.s.accb[(size_t)(3 + k) * N + i] : 0.0;
+        tdm[k] = damping ? d.s.accb[(size_t)(6 + k) * N + i] : 0.0;
     }
     // the wall stress of moving particles with a wall in their list, out of
     // line (its nine sums take registers only there); each sum still runs
@@ -3304,7 +3350,18 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
     REC(9);
     LAUNCH_ND(k_shepard_eos, nblk(N, tbk(d, TP_SHEPARD)), tbk(d, TP_SHEPARD), d); n++;
     REC(10);
-    LAUNCH_ND(k_strain, nblk(N, tbk(d, TP_STRAIN)), tbk(d, TP_STRAIN), d); n++;
+    const bool visc = sizeof(real) == 8 && d.p.visc;
+    {
+        const unsigned tb = tbk(d, TP_STRAIN), g = nblk(N, tb);
+        if (visc) {
+            if (d.p.ndim == 2) k_strain<2, 1><<<g, tb, 0, st>>>(d);
+            else k_strain<3, 1><<<g, tb, 0, st>>>(d);
+        } else {
+            if (d.p.ndim == 2) k_strain<2, 0><<<g, tb, 0, st>>>(d);
+            else k_strain<3, 0><<<g, tb, 0, st>>>(d);
+        }
+        n++;
+    }
     if (d.p.flagum == 1) { k_saturation<<<nblk(N, 128), 128, 0, st>>>(d); n++; }
     REC(11);
     if (regu) { LAUNCH_ND(k_regu, nblk(N, 128), 128, d, d.s.eps, d.s.eps_tmp, 1); n++; }
@@ -3340,11 +3397,29 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
     {
         const bool drag = d.p.fli > 1, vib = d.p.flv != 0;
         const dim3 g(nblk(N, tbk(d, TP_ACCEL_B))), b(tbk(d, TP_ACCEL_B));
+        // the own type's sums, where the strain pass did not take them; the
+        // drag's, in runs that have any
+        if (!visc) {
+            if (d.p.ndim == 2) {
+                if (vib) k_accel_b<2, 0, 0, 1><<<g, b, 0, st>>>(d);
+                else k_accel_b<2, 0, 0><<<g, b, 0, st>>>(d);
+            } else {
+                if (vib) k_accel_b<3, 0, 0, 1><<<g, b, 0, st>>>(d);
+                else k_accel_b<3, 0, 0><<<g, b, 0, st>>>(d);
+            }
+            n++;
+        }
+        if (d.p.fli >= 1) {
+            if (d.p.ndim == 2) {
+                if (drag) k_accel_b<2, 1, 1><<<g, b, 0, st>>>(d);
+                else k_accel_b<2, 0, 1><<<g, b, 0, st>>>(d);
+            } else {
+                if (drag) k_accel_b<3, 1, 1><<<g, b, 0, st>>>(d);
+                else k_accel_b<3, 0, 1><<<g, b, 0, st>>>(d);
+            }
+            n++;
+        }
         if (d.p.ndim == 2) {
-            if (vib) k_accel_b<2, 0, 0, 1><<<g, b, 0, st>>>(d);
-            else k_accel_b<2, 0, 0><<<g, b, 0, st>>>(d);
-            if (drag) k_accel_b<2, 1, 1><<<g, b, 0, st>>>(d);
-            else k_accel_b<2, 0, 1><<<g, b, 0, st>>>(d);
             if (vib) {
                 if (art) k_accel_b_tail<2, 1, 1><<<g, b, 0, st>>>(d);
                 else k_accel_b_tail<2, 0, 1><<<g, b, 0, st>>>(d);
@@ -3353,10 +3428,6 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
                 else k_accel_b_tail<2, 0><<<g, b, 0, st>>>(d);
             }
         } else {
-            if (vib) k_accel_b<3, 0, 0, 1><<<g, b, 0, st>>>(d);
-            else k_accel_b<3, 0, 0><<<g, b, 0, st>>>(d);
-            if (drag) k_accel_b<3, 1, 1><<<g, b, 0, st>>>(d);
-            else k_accel_b<3, 0, 1><<<g, b, 0, st>>>(d);
             if (vib) {
                 if (art) k_accel_b_tail<3, 1, 1><<<g, b, 0, st>>>(d);
                 else k_accel_b_tail<3, 0, 1><<<g, b, 0, st>>>(d);
@@ -3365,8 +3436,8 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
                 else k_accel_b_tail<3, 0><<<g, b, 0, st>>>(d);
             }
         }
+        n++;
     }
-    n += 3;
     REC(18);
     LAUNCH_ND(k_xsph_update, nblk(N, tbk(d, TP_XSPH)), tbk(d, TP_XSPH), d); n++;
     REC(19);
