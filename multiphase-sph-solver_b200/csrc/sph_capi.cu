@@ -273,6 +273,7 @@ void fill_dev_params(DevParams& p, const sphgpu_params* P)
     p.ninst = 0;
     p.split = p.ss_coupled ? 0 : 1;
     p.visc = 0;                        // set_visc
+    p.solids = 1;                      // update_static_params
     for (int q = 0; q < TP_COUNT; q++) p.tb[q] = 128;
     p.flr = P->flr == 1 ? 1 : 0;
     p.rain_lp = 0; p.rain_vrain = 0.0; p.rain_press = 0.0;
@@ -691,7 +692,11 @@ int first_vbx_wall(const sphgpu_ctx* c, int a, int b)
 void update_static_params(sphgpu_ctx* c)
 {
     const int w0 = first_vbx_wall(c, 0, c->N);
-    for (int p = 0; p < 2; p++) c->d[p].p.first_vbx_wall = w0;
+    const int solids = std::any_of(c->h_type.begin(), c->h_type.end(), [](int t) { return t == 2 || t == 4; });
+    for (int p = 0; p < 2; p++) {
+        c->d[p].p.first_vbx_wall = w0;
+        c->d[p].p.solids = solids;
+    }
     if (!c->h_inst.empty()) {
         for (InstGrid& g : c->h_inst) g.first_vbx_wall = first_vbx_wall(c, g.first, g.first + g.count);
         cuda_fail(c, cudaMemcpyAsync(c->d_inst, c->h_inst.data(), sizeof(InstGrid) * c->h_inst.size(),
@@ -1552,6 +1557,7 @@ int sphgpu_update_params(sphgpu_ctx* c, const sphgpu_params* P)
         const DevParams keep = dp;
         fill_dev_params(dp, P);
         dp.first_vbx_wall = keep.first_vbx_wall;
+        dp.solids = keep.solids;
         dp.bulk = keep.bulk;
         dp.cfl_on = keep.cfl_on; dp.cfl_c = keep.cfl_c; dp.cfl_f = keep.cfl_f;
         dp.rain_lp = keep.rain_lp; dp.rain_vrain = keep.rain_vrain; dp.rain_press = keep.rain_press;

@@ -90,6 +90,7 @@ struct DevParams {
     int ss_coupled;            // 1: coupled_Water_Soil_Structure (ss_type 1-3 with acc_type 2)
     double ss_myu, ss_zeta;
     int bulk;                  // 1: the FP32-bulk form (pair records in FP32)
+    int solids;                // 1: the context holds particles of type 2 or 4 (no pass makes any)
     int visc;                  // 1: the strain pass forms the artificial-viscosity sums (FP64 form; no
                                // damping, no vibration)
     int flts;                  // >= 1: TSSMP stress transformation around the soil models

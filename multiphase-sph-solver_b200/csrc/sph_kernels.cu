@@ -41,6 +41,7 @@
 // by both forms and lives in the FP64 build only.
 #include <cub/cub.cuh>
 #include <climits>
+#include <type_traits>
 #include "sph_device.cuh"
 #include "sph_constitutive.cuh"
 
@@ -65,14 +66,13 @@ namespace SPH_NS {
 #ifndef SPH_MINB
 #define SPH_MINB 4
 #endif
-// the constitutive pass keeps a dense 6x6 tangent per thread: 2 blocks of
-// 128 threads per SM leave it 222 registers and no spills
+// the constitutive pass: its solids' part (SPH_MINB_STRESS) and the others'
 #ifndef SPH_MINB_STRESS
-#define SPH_MINB_STRESS 2
+#define SPH_MINB_STRESS 4
 #endif
-// the momentum pass: its neighbour loops (k_accel_b) at 7 blocks per SM
-// (72 registers, a few spills: faster than 8, 6 or 5), its per-particle tail
-// (k_accel_b_tail) at 6 (faster than 5 and 4)
+#ifndef SPH_MINB_STRESSF
+#define SPH_MINB_STRESSF 6
+#endif
 #ifndef SPH_MINB_ACCB
 #define SPH_MINB_ACCB 6
 #endif
@@ -1164,12 +1164,22 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_saturation(Dev d)
 // PHASE 0 does all of it.  Where stress_regu can run (step_regu within the
 // run), PHASE 1 stops after the constitutive update (writing sig_next), the
 // smoothing pass runs, and PHASE 2 continues from the smoothed stresses.
-template <int ND, int PHASE>
-__global__ void __launch_bounds__(128, SPH_MINB_STRESS) k_stress(Dev d)
+//
+// SOLID 1 takes the solid particles (types 2 and 4), SOLID 0 the others, SOLID 2
+// all of them (the bulk form, which is built with multiply-adds contracted and
+// would contract other ones in the parts).  The
+// solids' dense 6 x 6 tangent takes all the registers it is given; fluids and
+// walls, more than half of a saturated soil and all of a dam break, need 72.
+// 4.45 M particles: 1.80 ms in one kernel at 2 blocks per SM (255 registers),
+// 1.56 ms as two, 1.16 ms with the solids at 4 (128 registers, 1 KB of spills; 3:
+// 1.26, 5: 1.12 but 2-D slopes 7% slower than at 4).
+template <int ND, int PHASE, int SOLID>
+__global__ void __launch_bounds__(128, SOLID == 2 ? 2 : SOLID ? SPH_MINB_STRESS : SPH_MINB_STRESSF) k_stress(Dev d)
 {
     const int i = IDX, N = d.p.N;
     if (i >= N || *d.s.err) return;
     const int ti = d.s.type[i], l = *d.s.step;
+    if (SOLID != 2 && (ti == 2 || ti == 4) != (SOLID == 1)) return;
     const double dt = step_dt(d);
     double s[6], ep[6], de[6], we9[9];
     for (int k = 0; k < 6; k++) {
@@ -1190,7 +1200,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRESS) k_stress(Dev d)
         we9[3] = w6[2]; we9[4] = 0.0; we9[5] = w6[3];
         we9[6] = w6[4]; we9[7] = w6[5]; we9[8] = 0.0;
     }
-    if (d.p.fli == 1 && ti == 2) {
+    if (SOLID && d.p.fli == 1 && ti == 2) {
         double cop = d.s.cop[i];
         const int pt = d.p.permtype;
         if (pt == 0) cop = d.s.s_cop[i];
@@ -1208,7 +1218,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRESS) k_stress(Dev d)
         }
         d.s.cop[i] = cop;
     }
-    if (ti == 1 || ti == 3) {
+    if (SOLID != 1 && (ti == 1 || ti == 3)) {
         double viscos1 = d.s.f_vis[i];
         if (ti == 1) {
             const double smin = d.s.f_smin[i];
@@ -1233,7 +1243,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRESS) k_stress(Dev d)
         dd_[3] = de[3]; dd_[4] = de[4]; dd_[5] = de[5];
         const double pr = d.s.pre[i];
         for (int a = 0; a < 6; a++) s[a] = (a < 3) ? -pr - viscos1 * dd_[a] : -viscos1 * dd_[a];
-    } else if (ti == 2 || ti == 4) {
+    } else if (SOLID != 0 && (ti == 2 || ti == 4)) {
         double D[6][6], adps[6] = {0, 0, 0, 0, 0, 0}, ds[6] = {0, 0, 0, 0, 0, 0};
         double erfs[6] = {0, 0, 0, 0, 0, 0};
         double dlam, dmu, sm;
@@ -1362,7 +1372,7 @@ __global__ void __launch_bounds__(128, SPH_MINB_STRESS) k_stress(Dev d)
         }
         return;
     }
-    if (PHASE == 2 && (ti == 2 || ti == 4)) {
+    if (PHASE == 2 && SOLID != 0 && (ti == 2 || ti == 4)) {
         vsig = d.s.vsig[i]; veps = d.s.veps[i]; divq = d.s.divq[i]; divr = d.s.divr[i];
         meps = d.s.meps[i];
         have_deq = true;
@@ -3366,22 +3376,30 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
     REC(11);
     if (regu) { LAUNCH_ND(k_regu, nblk(N, 128), 128, d, d.s.eps, d.s.eps_tmp, 1); n++; }
     REC(12);
-    if (regu) {
-        if (d.p.ndim == 2) k_stress<2, 1><<<nblk(N, tbk(d, TP_STRESS)), tbk(d, TP_STRESS), 0, st>>>(d);
-        else k_stress<3, 1><<<nblk(N, tbk(d, TP_STRESS)), tbk(d, TP_STRESS), 0, st>>>(d);
-    } else {
-        if (d.p.ndim == 2) k_stress<2, 0><<<nblk(N, tbk(d, TP_STRESS)), tbk(d, TP_STRESS), 0, st>>>(d);
-        else k_stress<3, 0><<<nblk(N, tbk(d, TP_STRESS)), tbk(d, TP_STRESS), 0, st>>>(d);
-    }
-    n++;
+    const unsigned sb = tbk(d, TP_STRESS), sg = nblk(N, sb);
+    auto stress = [&](auto phase) {
+        constexpr int PH = decltype(phase)::value;
+        if constexpr (sizeof(real) == 4) {
+            if (d.p.ndim == 2) k_stress<2, PH, 2><<<sg, sb, 0, st>>>(d);
+            else k_stress<3, PH, 2><<<sg, sb, 0, st>>>(d);
+            n++;
+            return;
+        }
+        if (d.p.solids) {
+            if (d.p.ndim == 2) k_stress<2, PH, 1><<<sg, sb, 0, st>>>(d);
+            else k_stress<3, PH, 1><<<sg, sb, 0, st>>>(d);
+            n++;
+        }
+        if (d.p.ndim == 2) k_stress<2, PH, 0><<<sg, sb, 0, st>>>(d);
+        else k_stress<3, PH, 0><<<sg, sb, 0, st>>>(d);
+        n++;
+    };
+    if (regu) stress(std::integral_constant<int, 1>());
+    else stress(std::integral_constant<int, 0>());
     REC(13);
     if (regu) { LAUNCH_ND(k_regu, nblk(N, 128), 128, d, d.s.sig_next, d.s.sig_tmp, 0); n++; }
     REC(14);
-    if (regu) {
-        if (d.p.ndim == 2) k_stress<2, 2><<<nblk(N, tbk(d, TP_STRESS)), tbk(d, TP_STRESS), 0, st>>>(d);
-        else k_stress<3, 2><<<nblk(N, tbk(d, TP_STRESS)), tbk(d, TP_STRESS), 0, st>>>(d);
-        n++;
-    }
+    if (regu) stress(std::integral_constant<int, 2>());
     REC(15);
     const bool art = d.p.art_stre_coe > 0.0;
     if (art) { LAUNCH_ND(k_art_rij, nblk(N, 128), 128, d); n++; }
