@@ -52,6 +52,7 @@ extern "C" int sphk_kl_synthesize(int n, int ndim, int K, int R, int no, int typ
                                   const int* nmode, const unsigned short* d_tidx);
 extern "C" int sphk_rf_cells(const int* ip, const double* dp, const double* d_xh, const int* d_type, int* d_cell,
                              int* d_count, int* d_err, cudaStream_t st);
+extern "C" size_t sphk_rf_matrix_doubles(size_t total);
 extern "C" int sphk_rf_factor(const int* ip, const double* dp, double* d_C, cudaStream_t st);
 extern "C" int sphk_rf_assign(const int* ip, const double* dp, const double* d_L, const double* d_zeta, double* d_E,
                               const int* d_cell, const int* d_type, double* d_out, cudaStream_t st);
@@ -2908,7 +2909,7 @@ int rf_run(sphgpu_ctx* c, const sphgpu_kl_domain* dom, const sphgpu_kl_field* fi
     const size_t off_out = off_E + 256 * ((8 * T + 255) / 256);
     const size_t off_C = off_out + 256 * ((8 * (size_t)N + 255) / 256);
     void* buf = nullptr;
-    CK(cudaMalloc(&buf, off_C + 8 * T * T));
+    CK(cudaMalloc(&buf, off_C + 8 * sphk_rf_matrix_doubles(T)));
     char* b = (char*)buf;
     int* d_cell = (int*)b;
     int* d_count = (int*)(b + off_count);

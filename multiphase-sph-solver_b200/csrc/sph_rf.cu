@@ -11,11 +11,11 @@
 // cell the cell's value.  Here every stage runs on the GPU:
 //   k_rf_cells   the cell of each particle and the per-cell counts (a cell of
 //                more than 39 particles is the reference's error 42)
-//   k_rf_corr    the correlation matrix, one thread per entry
-//   k_rf_diag    a 64 x 64 diagonal block factored in shared memory
-//   k_rf_panel   the rows below it solved against it
+//   k_rf_corr    the correlation matrix's lower triangle, one thread per entry
+//   k_rf_panel   a 64-column panel: its diagonal block factored, the rows below
+//                solved against it
 //   k_rf_update  the trailing lower triangle less the panel's outer product
-//                (64 x 64 output tiles from shared memory)
+//                (64 x 64 output tiles, FP64 tensor-core products)
 //   k_rf_gemv    E = L zeta, one warp per row
 //   k_rf_assign  each particle's value from its cell (normal or lognormal map
 //                with the depth trend, as the reference writes it)
@@ -68,7 +68,7 @@ __global__ void k_rf_cells(RFArgs a, const double* xh, const int* type, int* cel
 __global__ void k_rf_corr(RFArgs a, double* C)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
-    if (j >= a.total) return;
+    if (j > k) return;                       // the factorisation reads the lower triangle
     double xk[3], xj[3];
     centre(a, k, xk);
     centre(a, j, xj);
@@ -93,92 +93,158 @@ __global__ void k_rf_corr(RFArgs a, double* C)
     C[(size_t)k * a.total + j] = acf;
 }
 
-// the diagonal block [k0, k0 + bs) factored in place (lower triangle),
-// right-looking inside the block; the radicand floored at 1e-6
-__global__ void __launch_bounds__(RF_B) k_rf_diag(double* A, int n, int k0, int bs)
+// A panel: the diagonal block [k0, k0 + 64) factored (right-looking, the
+// radicand floored at 1e-6), and L[i][k0 .. k0 + 64) for the 64 rows below that
+// the block takes, by forward substitution.  Every block factors the diagonal
+// block for itself, in place of a launch of one block that the others wait
+// for.  Four threads hold a row, every fourth column each, in registers: a
+// step of either part is one column's quotients, then the multiply-adds of all
+// later columns, which are independent (a running sum per column is a chain of
+// 2,016).  Quotients by the pivot are taken from its reciprocal with one
+// correction step.  The factored block goes to `diag`, from where k_rf_update
+// puts it into the matrix (other blocks may still be reading the unfactored
+// one here).  Rows and columns past n read as the identity's.  Bound by
+// latency: 64 steps of a reciprocal root and two barriers, then 64 of a
+// broadcast and a quotient: 36 us a panel (45 with a square root and a
+// reciprocal each; 130 with one thread per row).
+__device__ __forceinline__ double rf_quotient(double x, double y, double ry)
 {
-    __shared__ double s[RF_B][RF_B + 1];
-    const int t = threadIdx.x;
-    for (int j = 0; j < bs; j++) s[t][j] = (t < bs) ? A[(size_t)(k0 + t) * n + k0 + j] : 0.0;
-    __syncthreads();
-    for (int k = 0; k < bs; k++) {
-        if (t == k) {
-            const double v = s[k][k];
-            s[k][k] = sqrt(v > 1.0e-6 ? v : 1.0e-6);
-        }
-        __syncthreads();
-        if (t > k && t < bs) s[t][k] = s[t][k] / s[k][k];
-        __syncthreads();
-        if (t > k && t < bs)
-            for (int j = k + 1; j <= t; j++) s[t][j] = s[t][j] - s[t][k] * s[j][k];
-        __syncthreads();
-    }
-    if (t < bs)
-        for (int j = 0; j < bs; j++) A[(size_t)(k0 + t) * n + k0 + j] = (j <= t) ? s[t][j] : 0.0;
+    const double q = x * ry;
+    return fma(fma(-q, y, x), ry, q);
 }
 
-// rows i >= k0 + bs of the panel: L[i][k0 .. k0 + bs) from the factored
-// diagonal block (forward substitution per row)
-__global__ void __launch_bounds__(128) k_rf_panel(double* A, int n, int k0, int bs)
+__global__ void __launch_bounds__(4 * RF_B) k_rf_panel(double* A, double* diag, int n, int k0)
 {
-    __shared__ double Lk[RF_B][RF_B + 1];
-    for (int e = threadIdx.x; e < bs * bs; e += blockDim.x) {
-        const int r = e / bs, c = e % bs;
-        Lk[r][c] = A[(size_t)(k0 + r) * n + k0 + c];
+    __shared__ double lt[RF_B][RF_B + 2];            // the factor, column by column
+    __shared__ double raw[2][RF_B];                  // the next column before its division, by turns
+    __shared__ double rec[RF_B];                     // the pivots' reciprocals
+    const int t = threadIdx.x, row = t >> 2, q = t & 3, lane = t & 31;
+    constexpr int U = RF_B / 4;
+    double x[U];                                     // columns 4 u + q
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int j = 4 * u + q;
+        const bool in = k0 + row < n && k0 + j < n;
+        x[u] = (in && j <= row) ? A[(size_t)(k0 + row) * n + k0 + j] : (j == row) ? 1.0 : 0.0;
+    }
+    if (q == 0) raw[0][row] = x[0];
+#pragma unroll
+    for (int k = 0; k < RF_B; k++) {
+        __syncthreads();
+        // the pivot's root and its reciprocal from one reciprocal root
+        const double v = raw[k & 1][k], f = v > 1.0e-6 ? v : 1.0e-6, r = rsqrt(f), p0 = f * r;
+        const double p = fma(fma(-p0, p0, f), 0.5 * r, p0);
+        const double l = (row == k) ? p : (row > k) ? rf_quotient(raw[k & 1][row], p, r) : 0.0;
+        if (q == 0) {
+            lt[k][row] = l;
+            if (row == k) rec[k] = r;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = (k + 1) / 4; u < U; u++) x[u] = fma(-l, lt[k][4 * u + q], x[u]);   // (columns up to k: unused)
+        if (k + 1 < RF_B && q == ((k + 1) & 3)) raw[(k + 1) & 1][row] = x[(k + 1) / 4];
     }
     __syncthreads();
-    const int i = k0 + bs + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double row[RF_B];
-    for (int k = 0; k < bs; k++) row[k] = A[(size_t)i * n + k0 + k];
-    for (int k = 0; k < bs; k++) {
-        double v = row[k];
-        for (int j = 0; j < k; j++) v = v - row[j] * Lk[k][j];
-        row[k] = v / Lk[k][k];
+    if (blockIdx.x == 0)
+        for (int e = t; e < RF_B * RF_B; e += 4 * RF_B) diag[e] = lt[e % RF_B][e / RF_B];
+    const int i = k0 + RF_B + blockIdx.x * RF_B + row;
+    if (k0 + RF_B >= n) {
+        // the last panel: one block, nobody else reads the matrix
+        for (int e = t; e < RF_B * RF_B; e += 4 * RF_B) {
+            const int a = e / RF_B, b = e % RF_B;
+            if (b <= a && k0 + a < n) A[(size_t)(k0 + a) * n + k0 + b] = lt[b][a];
+        }
+        return;
     }
-    for (int k = 0; k < bs; k++) A[(size_t)i * n + k0 + k] = row[k];
+    const double* src = A + (size_t)min(i, n - 1) * n + k0 + q;
+#pragma unroll
+    for (int u = 0; u < U; u++) x[u] = src[4 * u];
+#pragma unroll
+    for (int k = 0; k < RF_B; k++) {
+        const double mine = __shfl_sync(0xffffffffu, x[k / 4], (lane & ~3) | (k & 3));
+        const double xk = rf_quotient(mine, lt[k][k], rec[k]);
+        if (q == (k & 3)) x[k / 4] = xk;
+#pragma unroll
+        for (int u = k / 4; u < U; u++)
+            if (4 * u + q > k) x[u] = fma(-xk, lt[k][4 * u + q], x[u]);
+    }
+    if (i < n)
+#pragma unroll
+        for (int u = 0; u < U; u++) A[(size_t)i * n + k0 + q + 4 * u] = x[u];
 }
 
 // the trailing lower triangle, A[i][j] -= sum_k L[i][k] L[j][k] over the
-// panel's columns, for k0 + bs <= j <= i < n: 64 x 64 output tiles, the
-// panel's columns staged 16 at a time (k-major, one column of padding so the
-// transposing stores fall in distinct banks); each thread owns rows
-// tr + 16 p and columns tc + 16 q, so the tile reads and writes are 128-byte
-// runs
-__global__ void __launch_bounds__(256) k_rf_update(double* A, int n, int k0, int bs)
+// panel's 64 columns, for k0 + 64 <= j <= i < n: 64 x 64 output tiles, both
+// operands' panels staged whole in shared memory, the products on the FP64
+// tensor cores (mma.sync m8n8k4, the tensor form that takes FP64): eight warps
+// of 16 x 32 outputs, 2 x 4 products per four columns from six operand loads.
+// Rows are padded to 68 doubles: the four columns of eight rows then fall in
+// distinct banks.  Three blocks per SM (80 registers, a few spills): with two
+// the outputs' loads are not hidden.  One update of 4,766 rows: 20 us; 38 us
+// with multiply-adds on an 8 x 4 register block.  Whole call, 4,830 cells 20.0 ->
+// 7.8 ms, 13,230 cells 83 -> 68 ms, the error against 64 bits unchanged.
+#define RF_LD 68
+__global__ void __launch_bounds__(256, 3) k_rf_update(double* A, const double* diag, int n, int k0)
 {
-    const int r0 = k0 + bs + blockIdx.y * RF_B, c0 = k0 + bs + blockIdx.x * RF_B;
-    if (c0 > r0 + RF_B - 1 || r0 >= n) return;        // wholly above the diagonal
-    __shared__ double As[16][RF_B + 1], Bs[16][RF_B + 1];
-    const int tr = threadIdx.x / 16, tc = threadIdx.x % 16;
-    double acc[4][4];
-    for (int p = 0; p < 4; p++)
-        for (int q = 0; q < 4; q++) acc[p][q] = 0.0;
-    for (int kc = 0; kc < bs; kc += 16) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < 16 * RF_B; e += blockDim.x) {
-            const int k = e % 16, r = e / 16;
-            const bool in = kc + k < bs;
-            As[k][r] = (in && r0 + r < n) ? A[(size_t)(r0 + r) * n + k0 + kc + k] : 0.0;
-            Bs[k][r] = (in && c0 + r < n) ? A[(size_t)(c0 + r) * n + k0 + kc + k] : 0.0;
-        }
-        __syncthreads();
+    if (blockIdx.x == 0)
+        for (int e = threadIdx.x; e < RF_B * RF_B; e += 256)
+            if (e % RF_B <= e / RF_B) A[(size_t)(k0 + e / RF_B) * n + k0 + e % RF_B] = diag[e];
+
+    // tile (r, c), c <= r, of the trailing triangle, numbered row by row
+    int r = (int)((sqrtf(8.f * blockIdx.x + 1.f) - 1.f) * 0.5f);
+    while ((r + 1) * (r + 2) / 2 <= (int)blockIdx.x) r++;
+    while (r * (r + 1) / 2 > (int)blockIdx.x) r--;
+    const int c = blockIdx.x - r * (r + 1) / 2;
+    const int r0 = k0 + RF_B + r * RF_B, c0 = k0 + RF_B + c * RF_B;
+    extern __shared__ double sm[];
+    double* As = sm;
+    double* Bs = (r == c) ? sm : sm + RF_B * RF_LD;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int wr = (warp >> 1) * 16, wc = (warp & 1) * 32, g = lane >> 2, q = lane & 3;
+    // the outputs' present values, on their way while the operands are staged:
+    // accumulator rows g, columns 2 q and 2 q + 1 of each 8 x 8 product.  (Not
+    // what the products are added to: the small products' sum, subtracted once,
+    // loses less.)
+    double old[2][4][2], acc[2][4][2];
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            double a[4], b[4];
+    for (int m = 0; m < 2; m++)
 #pragma unroll
-            for (int p = 0; p < 4; p++) { a[p] = As[k][tr + 16 * p]; b[p] = Bs[k][tc + 16 * p]; }
+        for (int u = 0; u < 4; u++)
 #pragma unroll
-            for (int p = 0; p < 4; p++)
-#pragma unroll
-                for (int q = 0; q < 4; q++) acc[p][q] = fma(a[p], b[q], acc[p][q]);
-        }
+            for (int h = 0; h < 2; h++) {
+                const int i = r0 + wr + 8 * m + g, j = c0 + wc + 8 * u + 2 * q + h;
+                old[m][u][h] = (i < n && j <= i) ? A[(size_t)i * n + j] : 0.0;
+                acc[m][u][h] = 0.0;
+            }
+    for (int e = t; e < RF_B * RF_B; e += 256) {
+        const int row = e / RF_B, k = e % RF_B;
+        As[row * RF_LD + k] = (r0 + row < n) ? A[(size_t)(r0 + row) * n + k0 + k] : 0.0;
+        if (r != c) Bs[row * RF_LD + k] = (c0 + row < n) ? A[(size_t)(c0 + row) * n + k0 + k] : 0.0;
     }
-    for (int p = 0; p < 4; p++)
-        for (int q = 0; q < 4; q++) {
-            const int i = r0 + tr + 16 * p, j = c0 + tc + 16 * q;
-            if (i < n && j <= i) A[(size_t)i * n + j] = A[(size_t)i * n + j] - acc[p][q];
-        }
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < RF_B; k += 4) {
+        double a[2], b[4];
+#pragma unroll
+        for (int m = 0; m < 2; m++) a[m] = As[(wr + 8 * m + g) * RF_LD + k + q];
+#pragma unroll
+        for (int u = 0; u < 4; u++) b[u] = Bs[(wc + 8 * u + g) * RF_LD + k + q];
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                    : "+d"(acc[m][u][0]), "+d"(acc[m][u][1]) : "d"(a[m]), "d"(b[u]));
+    }
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int i = r0 + wr + 8 * m + g, j = c0 + wc + 8 * u + 2 * q + h;
+                if (i < n && j <= i) A[(size_t)i * n + j] = old[m][u][h] - acc[m][u][h];
+            }
 }
 
 // E = L zeta over the lower triangle, one warp per row
@@ -258,21 +324,22 @@ extern "C" int sphk_rf_cells(const int* ip, const double* dp, const double* d_xh
 
 // Stage 2: the correlation matrix of the cell centres into d_C (total x
 // total, row-major) and its lower Cholesky factor in place (the entries above
-// the diagonal are left undefined).
+// the diagonal are left undefined).  d_C has room for sphk_rf_matrix_doubles.
+extern "C" size_t sphk_rf_matrix_doubles(size_t total) { return total * total + RF_B * RF_B; }
+
 extern "C" int sphk_rf_factor(const int* ip, const double* dp, double* d_C, cudaStream_t st)
 {
     const RFArgs a = rf_args(ip, dp);
     const int T = a.total;
     k_rf_corr<<<dim3((T + 255) / 256, T), 256, 0, st>>>(a, d_C);
+    double* d_diag = d_C + (size_t)T * T;
+    const int smem = 2 * RF_B * RF_LD * (int)sizeof(double);
+    if (cudaFuncSetAttribute(k_rf_update, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 1;
     for (int k0 = 0; k0 < T; k0 += RF_B) {
-        const int bs = (T - k0) < RF_B ? (T - k0) : RF_B;
-        k_rf_diag<<<1, RF_B, 0, st>>>(d_C, T, k0, bs);
-        const int rest = T - k0 - bs;
-        if (rest > 0) {
-            k_rf_panel<<<(rest + 127) / 128, 128, 0, st>>>(d_C, T, k0, bs);
-            const int tiles = (rest + RF_B - 1) / RF_B;
-            k_rf_update<<<dim3(tiles, tiles), 256, 0, st>>>(d_C, T, k0, bs);
-        }
+        const int rest = T - k0 - RF_B;
+        const int tiles = (rest > 0) ? (rest + RF_B - 1) / RF_B : 0;
+        k_rf_panel<<<tiles > 0 ? tiles : 1, 4 * RF_B, 0, st>>>(d_C, d_diag, T, k0);
+        if (tiles > 0) k_rf_update<<<tiles * (tiles + 1) / 2, 256, smem, st>>>(d_C, d_diag, T, k0);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
