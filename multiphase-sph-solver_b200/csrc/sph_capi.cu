@@ -32,12 +32,14 @@ extern "C" int sphk_enqueue_physics(const Dev* d, cudaStream_t st, cudaEvent_t* 
 extern "C" int sphk_enqueue_physics_bulk32(const Dev* d, cudaStream_t st, cudaEvent_t* ev, int regu);
 extern "C" const char* const sphk_stage_names[];
 extern "C" size_t sphk_kl_sort_bytes(size_t total);
-extern "C" int sphk_kl_order(const double* d_r, int K, int ndim, double* keys_in, double* keys_out, uint32_t* vals_in,
-                             uint32_t* vals_out, void* sort_tmp, size_t sort_bytes, cudaStream_t st);
+extern "C" int sphk_kl_order(const double* d_r, int K, int ndim, size_t total, const uint32_t* list, double* keys_in,
+                             double* keys_out, uint32_t* vals_in, uint32_t* vals_out, void* sort_tmp,
+                             size_t sort_bytes, cudaStream_t st);
 extern "C" int sphk_kl_field(int n, int ndim, int K, int no, int type, const double* x_trans, double mean_value,
                              double sd_value, double coe_depth, double soil_max, double water_max, const double* d_xh,
                              const int* d_type, const void* d_terms, const double* d_sqrt_eig, const double* d_xi,
-                             double* d_out, cudaStream_t st);
+                             double* d_out, const void* d_modes, const int* nmode, const unsigned short* d_tidx,
+                             cudaStream_t st);
 extern "C" size_t sphk_order_temp_bytes(int N, int end_bit);
 extern "C" int sphk_order_sort(const Dev* dp, void* tmp, size_t bytes, int end_bit, unsigned long long* kin,
                                unsigned long long* kout, int* vin, int* vout, cudaStream_t st);
@@ -181,6 +183,10 @@ struct sphgpu_ctx {
     std::mutex out_mu;
     std::condition_variable out_cv;
     long out_ticket = 0, out_turn = 0;
+    // device scratch of the random-field calls, kept from one to the next
+    // while it is small (field_scratch)
+    void* fs[3] = {nullptr, nullptr, nullptr};
+    size_t fs_bytes[3] = {0, 0, 0};
     std::vector<InstGrid> h_inst;     // batched context: the instance table (empty: one system)
     InstGrid* d_inst = nullptr;
     // the re-sorted state (sphgpu_set_reorder): re-sort every reorder_every
@@ -1024,6 +1030,8 @@ void sphgpu_destroy(sphgpu_ctx* c)
     invalidate_graphs(c);
     for (void* p : c->allocs) cudaFree(p);
     if (c->perm_tmp) cudaFree(c->perm_tmp);
+    for (void* p : c->fs)
+        if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->mat_pinned) cudaFreeHost(c->mat_pinned);
     for (int b = 0; b < 2; b++) {
@@ -2567,16 +2575,15 @@ void kl_solve_wi(std::vector<double>& wi, const double a_x[3], const double rl[3
             double x1 = lo[i] + kKlPrec, x2 = up[i] - kKlPrec, xm, f1, fm;
             const bool odd = (i + 1) % 2 == 1;
             xm = odd ? (x1 + x2) * 0.5 : (x1 + x2) / 2.0;
+            // f at x1 is formed once: where x1 moves it takes the value at xm
+            auto f = [&](double x) {
+                return odd ? 2.0 / dira - x * std::tan(x * a) : 2.0 / dira * std::tan(x * a) + x;
+            };
+            f1 = f(x1);
             do {
-                if (odd) {
-                    f1 = 2.0 / dira - x1 * std::tan(x1 * a);
-                    fm = 2.0 / dira - xm * std::tan(xm * a);
-                } else {
-                    f1 = 2.0 / dira * std::tan(x1 * a) + x1;
-                    fm = 2.0 / dira * std::tan(xm * a) + xm;
-                }
+                fm = f(xm);
                 if ((f1 * fm) < 0.0) x2 = xm;
-                else x1 = xm;
+                else { x1 = xm; f1 = fm; }
                 xm = (x1 + x2) * 0.5;
             } while (std::fabs(fm) > kKlPrec);
             wi[(size_t)i * 3 + d] = xm;
@@ -2585,6 +2592,39 @@ void kl_solve_wi(std::vector<double>& wi, const double a_x[3], const double rl[3
 }
 
 struct HostKLTerm { double w, alpha; int use_cos; int pad; };
+
+// Device scratch of one random-field call, given back at its end.  Buffers of
+// up to 256 MB stay with the context for the next call (allocating and freeing
+// 190 MB took 2 of the 10 ms of a correlation-matrix field's call); larger ones
+// are freed.  Slots: 0 a plan's or field's small arrays, 1 the field's values, 2 the
+// correlation matrix and its vectors.
+struct FieldScratch {
+    sphgpu_ctx* c;
+    int slot;
+    char* p = nullptr;
+    FieldScratch(sphgpu_ctx* c_, int slot_) : c(c_), slot(slot_) {}
+    FieldScratch(const FieldScratch&) = delete;
+    int get(size_t bytes)
+    {
+        if (c->fs_bytes[slot] < bytes) {
+            if (c->fs[slot]) cudaFree(c->fs[slot]);
+            c->fs[slot] = nullptr;
+            c->fs_bytes[slot] = 0;
+            CK(cudaMalloc(&c->fs[slot], bytes));
+            c->fs_bytes[slot] = bytes;
+        }
+        p = static_cast<char*>(c->fs[slot]);
+        return 0;
+    }
+    ~FieldScratch()
+    {
+        if (c->fs_bytes[slot] > ((size_t)256 << 20)) {
+            cudaFree(c->fs[slot]);
+            c->fs[slot] = nullptr;
+            c->fs_bytes[slot] = 0;
+        }
+    }
+};
 
 // The expansion of one field: per term the selected 1-D root, normalisation
 // and parity on each axis, and sqrt(lambda); terms in the reference's order.
@@ -2606,23 +2646,50 @@ int kl_plan(sphgpu_ctx* c, const double a[3], const sphgpu_kl_field& f, int K, K
             const double w = wi[(size_t)i * 3 + d], dirac = f.rl_value[d];
             r[(size_t)i * 3 + d] = 4.0 * dirac / (4.0 + w * w * dirac * dirac);
         }
-    const size_t total = (nd == 2) ? (size_t)K * K : (size_t)K * K * K;
-    if (total > 0xffffffffull) return SPHGPU_E_ARG;
+    const size_t all = (nd == 2) ? (size_t)K * K : (size_t)K * K * K;
+    if (all > 0xffffffffull) return SPHGPU_E_ARG;
+    // The candidates.  Where every axis's eigenvalues do not increase with the
+    // index (the roots w do), a product at (m, n, k) comes after those at every
+    // smaller index triple: they are as large (a rounded product does not
+    // decrease with a factor) and have smaller linear indices, which order
+    // equal ones.  It can then be among the K largest only if there are fewer
+    // than K of them, (m + 1)(n + 1)(k + 1) <= K: 9,800 of 64 million for
+    // K = 400 in 3-D, where ordering all took 6 ms and 2.6 GB.
+    bool falling = true;
+    for (int d = 0; d < nd; d++)
+        for (int i = 0; i < K; i++) {
+            const double v = r[(size_t)i * 3 + d];
+            falling = falling && v > 0.0 && std::isfinite(v) && (i == 0 || v <= r[(size_t)(i - 1) * 3 + d]);
+        }
+    std::vector<uint32_t> list;
+    if (falling)
+        for (int m = 0; m < K; m++)
+            for (int n = 0; n < K / (m + 1); n++) {
+                if (nd == 2) list.push_back((uint32_t)m * K + n);
+                else
+                    for (int k = 0; k < K / ((m + 1) * (n + 1)); k++)
+                        list.push_back(((uint32_t)m * K + n) * K + k);
+            }
+    const size_t total = falling ? list.size() : all;
     const size_t sort_bytes = sphk_kl_sort_bytes(total);
-    void* buf = nullptr;
+    FieldScratch buf(c, 0);
     const size_t off_r = 0, off_ki = 256 * ((sizeof(double) * 3 * K + 255) / 256);
     const size_t off_ko = off_ki + 256 * ((8 * total + 255) / 256);
     const size_t off_vi = off_ko + 256 * ((8 * total + 255) / 256);
     const size_t off_vo = off_vi + 256 * ((4 * total + 255) / 256);
-    const size_t off_tmp = off_vo + 256 * ((4 * total + 255) / 256);
+    const size_t off_li = off_vo + 256 * ((4 * total + 255) / 256);
+    const size_t off_tmp = off_li + 256 * ((4 * list.size() + 255) / 256);
     const size_t bytes = off_tmp + sort_bytes;
-    CK(cudaMalloc(&buf, bytes));
-    char* b = (char*)buf;
+    if (const int e = buf.get(bytes)) return e;
+    char* b = buf.p;
     int rc = 0;
     do {
         if (cuda_fail(c, cudaMemcpyAsync(b + off_r, r.data(), sizeof(double) * 3 * K, cudaMemcpyHostToDevice, c->st),
                       "cudaMemcpyAsync")) { rc = SPHGPU_E_CUDA; break; }
-        if (sphk_kl_order((const double*)(b + off_r), K, nd, (double*)(b + off_ki), (double*)(b + off_ko),
+        if (falling && cuda_fail(c, cudaMemcpyAsync(b + off_li, list.data(), 4 * list.size(), cudaMemcpyHostToDevice,
+                                                    c->st), "cudaMemcpyAsync")) { rc = SPHGPU_E_CUDA; break; }
+        if (sphk_kl_order((const double*)(b + off_r), K, nd, total, falling ? (const uint32_t*)(b + off_li) : nullptr,
+                          (double*)(b + off_ki), (double*)(b + off_ko),
                           (uint32_t*)(b + off_vi), (uint32_t*)(b + off_vo), b + off_tmp, sort_bytes, c->st)) {
             rc = cuda_fail(c, cudaGetLastError(), "K-L eigenvalue ordering");
             if (!rc) rc = SPHGPU_E_CUDA;
@@ -2663,8 +2730,30 @@ int kl_plan(sphgpu_ctx* c, const double a[3], const sphgpu_kl_field& f, int K, K
             se[j] = std::sqrt(eig[j]);
         }
     } while (0);
-    cudaFree(buf);
     return rc;
+}
+
+// The distinct 1-D eigenfunctions of an expansion, axis by axis in order of
+// first use (nmode[d] of axis d): for each, the position in plan.terms of a
+// term factor that is it; and each term's factors among its axis's.
+std::vector<size_t> kl_modes(const KLPlan& plan, int K, int nd, int nmode[3], std::vector<unsigned short>& tidx)
+{
+    std::vector<size_t> at;
+    tidx.resize((size_t)K * nd);
+    for (int d = 0; d < 3; d++) nmode[d] = 0;
+    for (int d = 0; d < nd; d++) {
+        std::vector<int> slot(K, -1);
+        for (int j = 0; j < K; j++) {
+            const size_t e = (size_t)j * nd + d;
+            const int id = plan.ids[e];
+            if (slot[id] < 0) {
+                slot[id] = nmode[d]++;
+                at.push_back(e);
+            }
+            tidx[e] = (unsigned short)slot[id];
+        }
+    }
+    return at;
 }
 
 // One field of SpatialVariables_Generate_2D / _3D for the context's
@@ -2678,25 +2767,35 @@ int kl_one_field(sphgpu_ctx* c, const double a[3], const double x_trans[3], doub
     KLPlan plan;
     int rc = kl_plan(c, a, f, K, plan);
     if (rc) return rc;
-    void* buf = nullptr;
     const size_t off_se = 256 * ((sizeof(HostKLTerm) * plan.terms.size() + 255) / 256);
     const size_t off_xi = off_se + 256 * ((8 * (size_t)K + 255) / 256);
-    CK(cudaMalloc(&buf, off_xi + 8 * (size_t)K));
-    char* b = (char*)buf;
+    std::vector<HostKLTerm> modes;
+    std::vector<unsigned short> tidx;
+    int nmode[3];
+    for (const size_t e : kl_modes(plan, K, nd, nmode, tidx)) modes.push_back(plan.terms[e]);
+    const size_t off_md = off_xi + 256 * ((8 * (size_t)K + 255) / 256);
+    const size_t off_ti = off_md + 256 * ((sizeof(HostKLTerm) * modes.size() + 255) / 256);
+    FieldScratch buf(c, 0);
+    if (const int e = buf.get(off_ti + 2 * tidx.size())) return e;
+    char* b = buf.p;
     do {
         if (cuda_fail(c, cudaMemcpyAsync(b, plan.terms.data(), sizeof(HostKLTerm) * plan.terms.size(),
                                          cudaMemcpyHostToDevice, c->st), "cudaMemcpyAsync") ||
             cuda_fail(c, cudaMemcpyAsync(b + off_se, plan.sqrt_eig.data(), 8 * (size_t)K, cudaMemcpyHostToDevice,
                                          c->st), "cudaMemcpyAsync") ||
             cuda_fail(c, cudaMemcpyAsync(b + off_xi, xi, 8 * (size_t)K, cudaMemcpyHostToDevice, c->st),
+                      "cudaMemcpyAsync") ||
+            cuda_fail(c, cudaMemcpyAsync(b + off_md, modes.data(), sizeof(HostKLTerm) * modes.size(),
+                                         cudaMemcpyHostToDevice, c->st), "cudaMemcpyAsync") ||
+            cuda_fail(c, cudaMemcpyAsync(b + off_ti, tidx.data(), 2 * tidx.size(), cudaMemcpyHostToDevice, c->st),
                       "cudaMemcpyAsync")) { rc = SPHGPU_E_CUDA; break; }
         const DevState& s = c->d[c->parity].s;
         if (sphk_kl_field(count, nd, K, f.no, f.type, x_trans, f.mean_value, f.sd_value, f.coe_depth, soil_max,
                           water_max, s.xh + 4 * (size_t)first, s.type + first, b, (const double*)(b + off_se),
-                          (const double*)(b + off_xi), d_out + first, c->st)) { rc = SPHGPU_E_CUDA; break; }
+                          (const double*)(b + off_xi), d_out + first, b + off_md, nmode,
+                          (const unsigned short*)(b + off_ti), c->st)) { rc = SPHGPU_E_CUDA; break; }
         if (cuda_fail(c, cudaStreamSynchronize(c->st), "cudaStreamSynchronize")) { rc = SPHGPU_E_CUDA; break; }
     } while (0);
-    cudaFree(buf);
     return rc;
 }
 
@@ -2748,8 +2847,9 @@ int kl_run(sphgpu_ctx* c, const sphgpu_kl_domain* dom, const sphgpu_kl_field* fi
     const int nd = c->P.ndim, N = c->N;
     double a[3], xt[3], soil_max, water_max;
     if (kl_dom(nd, dom, a, xt, &soil_max, &water_max)) return 13;
-    double* d_out = nullptr;
-    CK(cudaMalloc(&d_out, sizeof(double) * N));
+    FieldScratch values(c, 1);
+    if (const int e = values.get(sizeof(double) * N)) return e;
+    double* d_out = reinterpret_cast<double*>(values.p);
     std::vector<double> v(N);
     int rc = 0;
     for (int q = 0; q < nfields && !rc; q++) {
@@ -2762,7 +2862,6 @@ int kl_run(sphgpu_ctx* c, const sphgpu_kl_domain* dom, const sphgpu_kl_field* fi
         if (out) std::memcpy(out + (size_t)q * N, v.data(), sizeof(double) * N);
         kl_store(c, fields[q].no, v.data(), 0, N);
     }
-    cudaFree(d_out);
     if (rc) return rc;
     return sphgpu_set_materials(c, c->h_fluid.empty() ? nullptr : c->h_fluid.data(),
                                 c->h_soil.empty() ? nullptr : c->h_soil.data(), N);
@@ -2780,8 +2879,9 @@ int sphgpu_kl_generate_batched(sphgpu_ctx* c, const sphgpu_kl_domain* doms, cons
     cudaSetDevice(c->device);
     if (const int ro = to_caller_order(c)) return ro;
     const int nd = c->P.ndim, N = c->N;
-    double* d_out = nullptr;
-    CK(cudaMalloc(&d_out, sizeof(double) * N));
+    FieldScratch values(c, 1);
+    if (const int e = values.get(sizeof(double) * N)) return e;
+    double* d_out = reinterpret_cast<double*>(values.p);
     int rc = 0;
     for (size_t q = 0; q < c->h_inst.size() && !rc; q++) {
         double a[3], xt[3], soil_max, water_max;
@@ -2795,7 +2895,6 @@ int sphgpu_kl_generate_batched(sphgpu_ctx* c, const sphgpu_kl_domain* doms, cons
         if (cuda_fail(c, cudaMemcpy(v.data(), d_out, sizeof(double) * N, cudaMemcpyDeviceToHost), "cudaMemcpy"))
             rc = SPHGPU_E_CUDA;
     }
-    cudaFree(d_out);
     if (rc) return rc;
     if (out) std::memcpy(out, v.data(), sizeof(double) * N);
     kl_store(c, f->no, v.data(), 0, N);
@@ -2908,9 +3007,9 @@ int rf_run(sphgpu_ctx* c, const sphgpu_kl_domain* dom, const sphgpu_kl_field* fi
     const size_t off_E = off_zeta + 256 * ((8 * T + 255) / 256);
     const size_t off_out = off_E + 256 * ((8 * T + 255) / 256);
     const size_t off_C = off_out + 256 * ((8 * (size_t)N + 255) / 256);
-    void* buf = nullptr;
-    CK(cudaMalloc(&buf, off_C + 8 * sphk_rf_matrix_doubles(T)));
-    char* b = (char*)buf;
+    FieldScratch buf(c, 2);
+    if (const int e = buf.get(off_C + 8 * sphk_rf_matrix_doubles(T))) return e;
+    char* b = buf.p;
     int* d_cell = (int*)b;
     int* d_count = (int*)(b + off_count);
     int* d_err = (int*)(b + off_err);
@@ -2949,7 +3048,6 @@ int rf_run(sphgpu_ctx* c, const sphgpu_kl_domain* dom, const sphgpu_kl_field* fi
                 cuda_fail(c, cudaStreamSynchronize(c->st), "cudaStreamSynchronize")) { rc = SPHGPU_E_CUDA; break; }
         }
     } while (0);
-    cudaFree(buf);
     return rc;
 }
 
@@ -3137,22 +3235,10 @@ int sphgpu_kl_synthesize(sphgpu_ctx* c, const sphgpu_kl_domain* dom, const sphgp
     std::vector<TCTerm> tc(plan.terms.size());
     for (size_t q = 0; q < tc.size(); q++)
         tc[q] = TCTerm{plan.terms[q].w, (float)plan.terms[q].alpha, plan.terms[q].use_cos};
-    // the separable form: per axis the distinct 1-D eigenfunctions the terms
-    // use (in order of first use) and each term's index among them
     std::vector<TCTerm> modes;
-    std::vector<unsigned short> tidx((size_t)K * nd);
-    int nmode[3] = {0, 0, 0};
-    for (int d = 0; d < nd; d++) {
-        std::vector<int> slot(K, -1);
-        for (int j = 0; j < K; j++) {
-            const int id = plan.ids[(size_t)j * nd + d];
-            if (slot[id] < 0) {
-                slot[id] = nmode[d]++;
-                modes.push_back(tc[(size_t)j * nd + d]);
-            }
-            tidx[(size_t)j * nd + d] = (unsigned short)slot[id];
-        }
-    }
+    std::vector<unsigned short> tidx;
+    int nmode[3];
+    for (const size_t e : kl_modes(plan, K, nd, nmode, tidx)) modes.push_back(tc[e]);
     const int Rc = R < 256 ? R : 256;   // realisations per launch
     const size_t off_se = 256 * ((sizeof(TCTerm) * tc.size() + 255) / 256);
     const size_t off_xi = off_se + 256 * ((8 * (size_t)K + 255) / 256);
@@ -3161,9 +3247,9 @@ int sphgpu_kl_synthesize(sphgpu_ctx* c, const sphgpu_kl_domain* dom, const sphgp
     const size_t off_err = off_cl + 256 * ((4 * (size_t)Rc * K + 255) / 256);
     const size_t off_md = off_err + 256;
     const size_t off_ti = off_md + 256 * ((sizeof(TCTerm) * modes.size() + 255) / 256);
-    void* buf = nullptr;
-    CK(cudaMalloc(&buf, off_ti + 2 * tidx.size() + 16));
-    char* b = (char*)buf;
+    FieldScratch buf(c, 0);
+    if (const int e = buf.get(off_ti + 2 * tidx.size() + 16)) return e;
+    char* b = buf.p;
     float total_ms = 0.f;
     do {
         if (cuda_fail(c, cudaMemcpyAsync(b, tc.data(), sizeof(TCTerm) * tc.size(), cudaMemcpyHostToDevice, c->st),
@@ -3203,7 +3289,6 @@ int sphgpu_kl_synthesize(sphgpu_ctx* c, const sphgpu_kl_domain* dom, const sphgp
             if (err) rc = err;
         }
     } while (0);
-    cudaFree(buf);
     if (kernel_ms) *kernel_ms = total_ms;
     return rc;
 }

@@ -106,6 +106,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
 __global__ void __launch_bounds__(KL_TILE_M, 1) k_kl_synth(KLTCArgs a)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
+    // the particles the field writes: of its phase.  A block without any (the
+    // particles of a phase mostly come one after another) only stores the
+    // others' NaN; in the other blocks their rows are zero.  Saturated soil
+    // column of 616,184 particles, 250,000 of them soil, 32 x 400: 2.39 ms with
+    // every row evaluated, 1.00 ms now; the call, its plan included, 10.7 -> 2.1 ms.
+    const int t = threadIdx.x, warp = t >> 5;
+    const int i = blockIdx.x * KL_TILE_M + t;
+    const bool live = i < a.n;
+    const int ptype = (live && !a.probe) ? a.ptype[i] : -1;
+    const bool soil_field = a.no >= 0 && a.no <= 3;
+    const bool writes = ptype == (soil_field ? 2 : 1);
+    if (!__syncthreads_or(writes || a.probe)) {
+        if (live)
+            for (int r = 0; r < a.R; r++) a.out[(size_t)r * a.n + i] = __int_as_float(0x7fc00000);
+        return;
+    }
     // layout: A_hi | A_lo | B_hi | B_lo | barrier | tmem base
     const int R = a.R;
     const uint32_t a_bytes = KL_TILE_M * KL_K_TILE * 4;
@@ -122,7 +138,6 @@ __global__ void __launch_bounds__(KL_TILE_M, 1) k_kl_synth(KLTCArgs a)
     const int nmodes = a.modes ? a.nmode[0] + a.nmode[1] + a.nmode[2] : 0;
     unsigned short* tix = reinterpret_cast<unsigned short*>(table + (size_t)nmodes * KL_TILE_M);
 
-    const int t = threadIdx.x, warp = t >> 5;
     int ncols = 32;
     while (ncols < R) ncols <<= 1;
 
@@ -140,8 +155,6 @@ __global__ void __launch_bounds__(KL_TILE_M, 1) k_kl_synth(KLTCArgs a)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
-    const int i = blockIdx.x * KL_TILE_M + t;
-    const bool live = i < a.n;
     double xa[3] = {0.0, 0.0, 0.0};
     double yp = 0.0;
     if (live) {
@@ -161,7 +174,7 @@ __global__ void __launch_bounds__(KL_TILE_M, 1) k_kl_synth(KLTCArgs a)
         for (int d = 0; d < a.ndim; d++)
             for (int m = 0; m < a.nmode[d]; m++) {
                 float v = 0.f;
-                if (live) {
+                if (writes) {
                     const KLTCTerm q = a.modes[a.moff[d] + m];
                     const double arg = q.w * xa[d];
                     const float red = (float)(arg - rint(arg * inv_two_pi_) * two_pi_);
@@ -195,7 +208,7 @@ __global__ void __launch_bounds__(KL_TILE_M, 1) k_kl_synth(KLTCArgs a)
         // this thread's Phi row for terms k0 .. k0 + kt
         for (int k = 0; k < KL_K_TILE; k++) {
             float phi = 0.f;
-            if (live && k < kt) {
+            if (writes && k < kt) {
                 phi = 1.f;
                 if (a.modes) {
                     for (int d = 0; d < a.ndim; d++)
@@ -263,9 +276,6 @@ __global__ void __launch_bounds__(KL_TILE_M, 1) k_kl_synth(KLTCArgs a)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok && !a.probe) {
         // epilogue: warp w holds accumulator lanes 32 w .. 32 w + 31 (particle t)
-        const int ptype = live ? a.ptype[i] : -1;
-        const bool soil_field = a.no >= 0 && a.no <= 3;
-        const bool writes = live && ((soil_field && ptype == 2) || (!soil_field && ptype == 1));
         double mean = 0.0, sigma = 0.0;
         if (writes) {
             mean = a.mean_value + ((ptype == 2 ? a.soil_max : a.water_max) - yp) * a.coe_depth;

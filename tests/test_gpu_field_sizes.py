@@ -1,11 +1,12 @@
 """Random fields at the sizes where their kernels change: correlation matrices
-around whole panels of the factorisation."""
+around whole panels of the factorisation, K-L expansions of few and of very
+many distinct factors, and fields of a phase that few or no particles have."""
 import numpy as np
 import pytest
 
 import scenes
 import sphgpu
-from checkers import rf_oracle
+from checkers import kl_oracle, rf_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -41,4 +42,41 @@ def test_matrices_around_whole_panels(cells, crest, ndx):
     err, want, n = rf_oracle(2, sc.xp, sc.ptype, sc.dr, f, d, z)
     assert err == 0 and n == cells
     _close(eng.rf_generate(dom, [sphgpu.kl_field(1, 2, 10.0e3, 3.0e3, [3.0, 0.8, 0.0], 100.0)], fl, z[None])[0], want)
+    eng.close()
+
+
+@pytest.mark.parametrize("ndim,K,rl", [
+    (2, 1, (6.0, 1.5, 0.0)), (2, 40, (1.0, 1.0, 0.0)), (2, 300, (0.05, 1.0, 0.0)),
+    (3, 1, (0.5, 0.25, 0.25)), (3, 56, (0.3, 0.3, 0.3)), (3, 64, (0.1, 1.0, 1.0)),
+])
+def test_expansions_of_few_and_many_factors(ndim, K, rl):
+    sc = scenes.slope_2d(H=1.0, dx=0.1) if ndim == 2 else scenes.soil_column_3d(dx=0.1)
+    eng, d, dom = _engine(sc)
+    xi = np.random.default_rng(K).standard_normal(K)
+    f = {"no": 0, "type": 1, "mean": 30.0, "sd": 3.0, "rl": list(rl), "coe_depth": 0.5}
+    want = kl_oracle(ndim, sc.xp, sc.ptype, f, d, xi, K)[0]
+    got = eng.kl_generate(dom, [sphgpu.kl_field(0, 1, 30.0, 3.0, list(rl), 0.5)], xi[None], K)[0]
+    _close(got, want)
+    eng.close()
+
+
+@pytest.mark.parametrize("no", (0, 4))
+def test_synthesis_of_one_phase(no):
+    """The tensor-core synthesis against the FP64 field, for a phase of part of
+    the particles and for one of none (every value NaN)."""
+    import torch
+    sc = scenes.soil_column_3d(dx=0.0625, with_water=False)
+    eng, d, dom = _engine(sc)
+    K, R = 40, 16
+    xi = np.random.default_rng(5).standard_normal((R, K))
+    field = sphgpu.kl_field(no, 1, 30.0, 3.0, [0.5, 0.3, 0.2], 2.0)
+    out = torch.full((R, eng.n), 7.0, dtype=torch.float32, device="cuda")
+    eng.kl_synthesize(dom, field, xi, out.data_ptr(), K)
+    got = out.cpu().numpy()
+    phase = sc.ptype == (2 if no == 0 else 1)
+    assert np.array_equal(np.isnan(got), np.broadcast_to(~phase, got.shape))
+    if phase.any():
+        for r in (0, R - 1):
+            want = eng.kl_generate(dom, [field], xi[r:r + 1], K)[0]
+            assert np.abs(got[r, phase] - want[phase]).max() <= 1e-5 * np.abs(want[phase]).max()
     eng.close()
