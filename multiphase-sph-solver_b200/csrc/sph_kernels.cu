@@ -138,20 +138,29 @@ __device__ __forceinline__ int cell_link(const CellGrid& g, int c, int slot)
     return (v <= 0 || v > g.ctotal) ? 0 : v + g.base;
 }
 
-// The rows of one group of particle i's list, in list order, the next row's
-// word loaded one row ahead.  A pass that sums over some of a group's types
+// The rows of one group of particle i's list, in list order, the words loaded
+// AHEAD rows (1 or 2) before their use.  Two rows pay where a row's own work is
+// a load or two, as in the Shepard pass (4.45 M particles 0.66 -> 0.56 ms,
+// 616,184 particles 0.107 -> 0.088); the strain and density passes, whose row
+// work hides one word's latency, lose to the second word's registers (2.87 ->
+// 2.95 and 1.49 -> 1.52 ms), and the others are unchanged.  A pass that sums over some of a group's types
 // skips the rows of the others; away from walls a group has one type, so the
 // lanes of a warp run row by row together on consecutive words and records.
-struct RowIter {
-    const int* p;              // the word after the prefetched one's
+template <int AHEAD>
+struct Rows {
+    const int* p;              // the last prefetched word's
     ptrdiff_t step;            // words from one row to the next: N, or -N in group B
-    size_t off;                // r * N + i of the prefetched row
-    int left, w1;
-    __device__ __forceinline__ RowIter(const Dev& d, int i, int n, int row0, int dir)
+    size_t off;                // r * N + i of the next row
+    int left, w1, w2;
+    __device__ __forceinline__ Rows(const Dev& d, int i, int n, int row0, int dir)
         : step(dir * (ptrdiff_t)d.p.N), off((size_t)row0 * d.p.N + i), left(n)
     {
         p = d.s.nbr + off;
         w1 = (n > 0) ? *p : 0;
+        if (AHEAD == 2) {
+            p += step;
+            w2 = (n > 1) ? *p : w1;
+        }
     }
     // the next row's particle, type code and offset; false past the last
     __device__ __forceinline__ bool next(int& j, int& tj, size_t& o)
@@ -161,12 +170,19 @@ struct RowIter {
         j = w1 >> 3;
         tj = w1 & 7;
         o = off;
-        off += step;
         p += step;
-        if (left > 0) w1 = *p;
+        if (AHEAD == 2) {
+            if (left > 0) off += step;
+            w1 = w2;
+            if (left > 1) w2 = *p;
+        } else {
+            off += step;
+            if (left > 0) w1 = *p;
+        }
         return true;
     }
 };
+using RowIter = Rows<1>;
 __device__ __forceinline__ RowIter rows_a(const Dev& d, int i) { return RowIter(d, i, d.s.nab[i] & 0xff, 0, 1); }
 // group B, or the whole list where it is not split
 __device__ __forceinline__ RowIter rows_b(const Dev& d, int i)
@@ -902,7 +918,7 @@ __global__ void __launch_bounds__(128, SPH_MINB) k_shepard_eos(Dev d)
     Sum<real> sup, sdown;
     const PairI<real> I = pair_i<ND, real>(d, i);
     const real rra = real(1.0) / I.h;
-    RowIter it = rows_a(d, i);
+    Rows<2> it(d, i, d.s.nab[i] & 0xff, 0, 1);
     int j, tj;
     size_t o;
     while (it.next(j, tj, o)) {
