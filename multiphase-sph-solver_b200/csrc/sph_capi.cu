@@ -750,7 +750,7 @@ struct RecMember {
 };
 constexpr int kMaxRecMembers = 48;
 constexpr int kRecChunk = 65536;          // records per staged chunk
-// particles per host thread of a download, up to 16 threads: 15,312 particles
+// particles per host thread of a download, up to 16 threads: 14,978 particles
 // take 0.8 ms with 2,048, 0.9 with 1,024 or 4,096, 1.1 with 8,192
 constexpr int kRecShare = 2048;
 
@@ -1494,7 +1494,7 @@ int sphgpu_download_particles(sphgpu_ctx* c, void* particles, int n, size_t stri
     // each record is read from pinned memory and written to the caller's.  One
     // chunk at a time on one stream, with threads started for its records and
     // the table copied to the device per call, took 0.25 ms for 1,358
-    // particles, 1.5 for 15,312 and 17.3 for 616,184; now 0.15, 0.8 and 15.0.
+    // particles, 1.5 for 14,978 and 17.3 for 616,184; now 0.15, 0.8 and 15.0.
     unsigned T = std::thread::hardware_concurrency();
     T = std::max(1u, std::min({T, 16u, (unsigned)((n + kRecShare - 1) / kRecShare)}));
     const int piece = kRecChunk / (int)T & ~31;          // records of one thread's part of a staging buffer
