@@ -2946,6 +2946,7 @@ __global__ void __launch_bounds__(128) k_free_solid(Dev d)
 // 507-629): the stress divergence between structure and soil / water pairs
 // with plain stresses (a water particle with a structure neighbour takes the
 // difference form); k_accel_b adds each row sum after the wall stress.
+template <int ND>
 __global__ void __launch_bounds__(128) k_coupled(Dev d)
 {
     const int i = IDX, N = d.p.N;
@@ -2964,7 +2965,7 @@ __global__ void __launch_bounds__(128) k_coupled(Dev d)
         const bool minus = (ti == 1 && tj == 4);
         if (!(plus || minus)) continue;
         real wr[3];
-        load_g<3, real>(d, o, wr);
+        load_g<ND, real>(d, o, wr);    // 2-D records have no z plane
         const double w[3] = {wr[0], wr[1], wr[2]};
         const double mj = d.s.mass[j], rj = d.s.rho[j];
         double sj[6], a[6], b[6];
@@ -3422,7 +3423,7 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
     REC(16);
     LAUNCH_ND(k_accel_a, nblk(N, tbk(d, TP_ACCEL_A)), tbk(d, TP_ACCEL_A), d); n++;
     if (d.p.flbndy == 5) { LAUNCH_ND(k_free_solid, nblk(N, 128), 128, d); n++; }
-    if (d.p.ss_coupled) { k_coupled<<<nblk(N, 128), 128, 0, st>>>(d); n++; }
+    if (d.p.ss_coupled) { LAUNCH_ND(k_coupled, nblk(N, 128), 128, d); n++; }
     if (d.p.ss_type >= 1) {
         LAUNCH_ND(k_ss_pair, nblk(N, 128), 128, d); n++;
         k_ss_struct<<<nblk(N, 128), 128, 0, st>>>(d); n++;
