@@ -162,6 +162,7 @@ struct sphgpu_ctx {
     std::vector<sphgpu_soil, UninitAlloc<sphgpu_soil>> h_soil;      // (K-L fields rewrite members)
     double* mat_pinned = nullptr;     // pinned, 4N: the per-particle material constants set_materials uploads
     int part_done = 0;     // parts of step l run through the method entries: 1 parttocell, 2 partisearching
+    int list_split = 0, list_bulk = 0;   // the form (DevParams::split, bulk) of the lists partisearching left
     sphgpu_rain rain = {};            // the rainfall record (flr 1), nrain as last set
     bool rain_set = false;
     sphgpu_vibration vib = {};        // the vibration table (flv 1, 2) as last set
@@ -1579,7 +1580,11 @@ int run_parts(sphgpu_ctx* c, int upto)
     if (c->part_done < 1 && upto >= 1) parts |= 1;
     if (c->part_done < 2 && upto >= 2) parts |= 2;
     if (upto >= 3) parts |= 4;
+    // the contact or precision form may have been set since the search: the
+    // passes read the lists in the form of now
+    if (c->part_done >= 2 && (d->p.split != c->list_split || d->p.bulk != c->list_bulk)) parts |= 2;
     if (parts) sphk_enqueue_nnps_parts(d, c->st, nullptr, parts);
+    if (parts & 2) { c->list_split = d->p.split; c->list_bulk = d->p.bulk; }
     if (upto >= 3) {
         if (!c->regu && c->l_host % c->P.step_regu == 0) { c->regu = true; invalidate_graphs(c); }
         set_visc(c);
@@ -2387,9 +2392,12 @@ int sphgpu_nnps(sphgpu_ctx* c, int* ninflu, int* influ)
     }
     if (c->part_done >= 2 && err == 0) {
         // the lists of the step that sphgpu_update will complete
-        sphk_enqueue_nnps_parts(&c->d[c->parity], c->st, nullptr, 2);
+        const Dev& d = c->d[c->parity];
+        sphk_enqueue_nnps_parts(&d, c->st, nullptr, 2);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(c->st));
+        c->list_split = d.p.split;
+        c->list_bulk = d.p.bulk;
     }
     return err;
 }

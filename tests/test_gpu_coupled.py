@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import scenes
-from checkers import STATE_FIELDS
+from checkers import ORC_JACOBI, ORC_POW_CR, STATE_FIELDS, Oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +39,70 @@ def test_switch_to_the_bulk_form(ndim, tmp_path):
     assert np.isfinite(a.get_field("vx")).all()
     a.close()
     b.close()
+
+
+def _wet_footing(ndim, ss):
+    """Soil with pore water, a footing and walls, all with stress and motion."""
+    sc = _coupled_footing(ndim)
+    soil = sc.ptype == 2
+    m = int(soil.sum())
+    for k, v in (("xp", sc.xp[soil]), ("vxp", np.zeros((m, 3))), ("ptype", np.full(m, 1, np.int32)),
+                 ("matype", np.zeros(m, np.int32)), ("permtype", np.zeros(m, np.int32)), ("etype", np.ones(m, np.int32))):
+        setattr(sc, k, np.concatenate([getattr(sc, k), v]))
+    sc.flags["fli"] = 1
+    sc.soils[2]["eps0"] = 0.6667             # porous: the water's porosity is the soil's
+    sc.problem.update(interc=1.0, pers=1.0e-4, perl=1.0e-4, perm=1.0e-4, ss=ss)
+    st = scenes.initialise(sc)
+    rng = np.random.default_rng(ndim)
+    solid = (st.fields["type"] == 2) | (st.fields["type"] == 4)
+    flat = (1.0, 1.0, float(ndim == 3))
+    st.fields["vxp"] = st.fields["vxp"] + 0.05 * (st.fields["type"] > 0)[:, None] * rng.standard_normal((sc.n, 3)) * flat
+    sig = np.where(solid[:, None], -1.0e3 * rng.random((sc.n, 6)), 0.0)
+    if ndim == 2:
+        sig[:, 4:] = 0.0
+    st.fields["sig"] = sig
+    return st
+
+
+@pytest.mark.parametrize("ndim", (2, 3))
+@pytest.mark.parametrize("before,after", (((0, 0.0, 0.0, 0), (2, 0.3, 0.1, 2)), ((2, 0.3, 0.1, 2), (2, 0.3, 0.1, 0)),
+                                          ((2, 0.3, 0.1, 0), (1, 0.3, 0.1, 2))))
+def test_contact_set_between_search_and_update(ndim, before, after):
+    """The contact form is read by update alone: setting it after the search
+    of a step (as the reference's classes do in the first one) gives the step of
+    a run that had it from the start."""
+    import sphgpu
+    st, want = _wet_footing(ndim, before), _wet_footing(ndim, after)
+    orc = Oracle(want.params, ORC_JACOBI, ORC_POW_CR)
+    orc.load_state(want.fields, want.fluid, want.soil)
+    eng = sphgpu.Engine(st.params, device=0)
+    eng.load_state(st.fields, st.fluid, st.soil)
+    assert eng.parttocell() == 0 and eng.partisearching() == 0
+    eng.update_params(want.params)
+    assert eng.update() == 0
+    eng.step(1)
+    assert orc.step(2) == 0
+    for f in STATE_FIELDS:
+        a, b = eng.get_field(f), orc.get_field(f)
+        assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f"), f
+    assert np.isfinite(orc.get_field("vx")).all()
+    eng.close()
+
+
+def test_precision_set_between_search_and_update():
+    import sphgpu
+    st = _wet_footing(2, (2, 0.3, 0.1, 2))
+    out = []
+    for late in (False, True):
+        eng = sphgpu.Engine(st.params, device=0)
+        eng.load_state(st.fields, st.fluid, st.soil)
+        if not late:
+            eng.set_precision(sphgpu.PREC_FP32_BULK)
+        assert eng.parttocell() == 0 and eng.partisearching() == 0
+        if late:
+            eng.set_precision(sphgpu.PREC_FP32_BULK)
+        assert eng.update() == 0
+        out.append([eng.get_field(f) for f in STATE_FIELDS])
+        eng.close()
+    for f, a, b in zip(STATE_FIELDS, *out):
+        assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f"), f
