@@ -689,6 +689,41 @@ void set_visc(sphgpu_ctx* c)
     invalidate_graphs(c);
 }
 
+// The bounds of h the search decides its candidates by (DevState::hb): over
+// the particles in the calculation, and dr where rain will join them (rainpro
+// gives it that h).  Only the speed of the search depends on them: a particle
+// outside takes FP64 tests.
+__global__ void k_h_bounds_start(Dev d)
+{
+    const bool rain = d.p.flr != 0;
+    d.s.hb[0] = rain ? (float)d.p.dr : __int_as_float(0x7f800000);
+    d.s.hb[1] = rain ? (float)d.p.dr : 0.f;
+}
+__global__ void __launch_bounds__(256) k_h_bounds(Dev d)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int lo = 0x7f800000, hi = 0;
+    if (i < d.p.N && d.s.type[i] != 7) {
+        const float h = (float)d.s.xh[4 * (size_t)i + 3];
+        if (h > 0.f && h <= 3.4028235e38f) lo = hi = __float_as_int(h);    // (positive values order as their bits)
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0 && hi != 0) {
+        atomicMin(reinterpret_cast<int*>(d.s.hb), lo);
+        atomicMax(reinterpret_cast<int*>(d.s.hb) + 1, hi);
+    }
+}
+// on the context's stream, after h or the types were set
+int update_h_bounds(sphgpu_ctx* c)
+{
+    const Dev& d = c->d[c->parity];
+    k_h_bounds_start<<<1, 1, 0, c->st>>>(d);
+    k_h_bounds<<<(c->N + 255) / 256, 256, 0, c->st>>>(d);
+    CK(cudaGetLastError());
+    return 0;
+}
+
 // the first wall (index order) with matype > 2 in [a, b), or b
 int first_vbx_wall(const sphgpu_ctx* c, int a, int b)
 {
@@ -970,6 +1005,7 @@ sphgpu_ctx* sphgpu_create(const sphgpu_params* P, int device)
     r |= dalloc(c, &s.s_ann, N); r |= dalloc(c, &s.s_zmf, N); r |= dalloc(c, &s.s_ramda, N); r |= dalloc(c, &s.s_sme0, N);
     r |= dalloc(c, &s.s_yalf, N); r |= dalloc(c, &s.s_ykap, N); r |= dalloc(c, &s.s_yalf_dil, N);
     r |= dalloc(c, &s.xh, 4 * (size_t)N); r |= dalloc(c, &s.xh_next, 4 * (size_t)N); r |= dalloc(c, &s.xs, 4 * (size_t)N); r |= dalloc(c, &s.xsf, 4 * (size_t)N); r |= dalloc(c, &s.xsp, 3 * (size_t)SPH_XSP_STRIDE(N));
+    r |= dalloc(c, &s.hb, 2);
     r |= dalloc(c, &s.de, 6 * (size_t)N); r |= dalloc(c, &s.we, 6 * (size_t)N); r |= dalloc(c, &s.color, N);
     r |= dalloc(c, &s.sr, 8 * (size_t)N);
     r |= dalloc(c, &s.eps_tmp, 6 * (size_t)N); r |= dalloc(c, &s.sig_tmp, 6 * (size_t)N);
@@ -1141,8 +1177,10 @@ int sphgpu_set_field(sphgpu_ctx* c, const char* name, const void* host, size_t c
         } else {
             for (int i = 0; i < N; i++) rec[(size_t)i * 4 + 3] = h[i];
         }
-        CK(cudaMemcpy(xh, rec.data(), sizeof(double) * rec.size(), cudaMemcpyHostToDevice));
-        return 0;
+        CK(cudaMemcpyAsync(xh, rec.data(), sizeof(double) * rec.size(), cudaMemcpyHostToDevice, c->st));
+        int r = (nc == 1) ? update_h_bounds(c) : 0;
+        CK(cudaStreamSynchronize(c->st));
+        return r;
     }
     const size_t esz = f->is_int ? 4 : 8;
     int r = ensure_pinned(c, count * esz);
@@ -1162,8 +1200,9 @@ int sphgpu_set_field(sphgpu_ctx* c, const char* name, const void* host, size_t c
     void* dst = field_ptr(c, name);
     if (!dst) return SPHGPU_E_ARG;
     CK(cudaMemcpyAsync(dst, c->pinned, count * esz, cudaMemcpyHostToDevice, c->st));
+    r = (std::strcmp(name, "type") == 0) ? update_h_bounds(c) : 0;
     CK(cudaStreamSynchronize(c->st));
-    return 0;
+    return r;
 }
 
 int sphgpu_get_field(sphgpu_ctx* c, const char* name, void* host, size_t count)
@@ -1437,7 +1476,7 @@ int sphgpu_upload_particles(sphgpu_ctx* c, const void* particles, int n, size_t 
     r = push_records(c, base, n, stride, tab);
     if (r) return r;
     update_static_params(c);
-    return 0;
+    return update_h_bounds(c);
 }
 
 int sphgpu_download_particles(sphgpu_ctx* c, void* particles, int n, size_t stride)

@@ -148,6 +148,8 @@ struct DevState {
     float *xsf;                // xs as FP32 records (x - xmin, y - ymin, z - zmin, word), word the particle
                                // index << 3 | its type code (the type for types 0-4, else 7) as bits
     float *xsp;                // its x, y, z as planes of SPH_XSP_STRIDE(N) values: the scan's tests
+    float *hb;                 // the smallest and the largest h (FP32) of the particles in the calculation, as
+                               // set: the scan's bounds
     // dynamic state
     double *vx;                // velocity after the step
     double *vx_next;           // per particle (vx x, y, z before XSPH, mass): one 32-byte record

@@ -420,10 +420,11 @@ __global__ void k_cellrange(Dev d)
     const Pos r = load_pos(d.s.xh, pid);
     store_pos(d.s.xs, q, r);
     // the search's FP32 records with the index-and-type word, and its planes;
-    // a candidate whose h is not dr has NaN for x, which no bound decides, so
-    // it takes the FP64 test
+    // a candidate whose h lies outside the context's bounds (or is not a
+    // number) has NaN for x, which no bound decides, so it takes the FP64 test
     float4 f = make_float4((float)(r.x - g.xmin), (float)(r.y - g.ymin), (float)(r.z - g.zmin), __int_as_float(w));
-    if ((float)r.h != (float)d.p.dr) f.x = __int_as_float(0x7fffffff);
+    const float hj = (float)r.h;
+    if (!(hj >= d.s.hb[0] && hj <= d.s.hb[1])) f.x = __int_as_float(0x7fffffff);
     reinterpret_cast<float4*>(d.s.xsf)[q] = f;
     const size_t NP = (size_t)SPH_XSP_STRIDE(N);
     d.s.xsp[q] = f.x;
@@ -431,23 +432,6 @@ __global__ void k_cellrange(Dev d)
     d.s.xsp[2 * NP + q] = f.z;
 }
 
-// partisearching (CPP_3-NNPS.cpp:265-374): neighbours of i in stencil order,
-// descending index inside each cell; inclusion dst <= h_i + h_j decided as the
-// reference decides it (sqrt of the FP64 sum of squares).
-//
-// Each candidate is first tested in FP32 on the (x - xmin, y - ymin, z - zmin,
-// h) records, against a margin M that bounds every rounding between the FP32
-// squared distance d2f and the exact one: the coordinates' rounding to FP32
-// (at most 2^-24 |coordinate|, and |x_j - xmin| <= |x_i - xmin| + |x_i - x_j|),
-// the subtraction, squares and sum, and the rounding of T = h_i + h_j and T^2.
-// With F_i the particle's largest |coordinate - min| and e = 2.2 u (F_i + 2 T),
-// u = 2^-24, every candidate with d2f <= 4 T^2 has |d2f - d2| <= nd e (4 T + e)
-// + 12.4 u T^2; M adds 32 u T^2 on top of that.  Candidates with d2f > 4 T^2
-// are outside whenever h_i > 10 u F_i (the error then grows more slowly than
-// d2f - T^2); the test requires h_i > 64 u F_i and otherwise sends every
-// candidate to the FP64 path.  Only candidates within M of T^2 take the FP64
-// path, where the sqrt is evaluated only within 1e-10 of the squared radius,
-// so the decisions are those of the reference.
 // The FP64 inclusion test of one candidate, as partisearching decides it:
 // sqrt of the FP64 sum of squares against h_i + h_j, the sqrt evaluated only
 // within 1e-10 of the squared radius (outside that band the comparison of the
@@ -465,25 +449,35 @@ __device__ __forceinline__ bool nnps_in_fp64(const double xi[3], double hi, cons
     return sqrt(d2) <= T;
 }
 
-// The decision bounds of a particle's candidates, all of h equal to its own:
-// inside below lo, outside above hi, in FP64 between.
+// The rounding margin M and the square of the radius Tf = h_i + h_j
 template <int ND>
-__device__ __forceinline__ void prefilter_bounds(float fh, float ce, float* lo, float* hi)
+__device__ __forceinline__ float prefilter_margin(float Tf, float ce, float* T2)
 {
     constexpr float U = 5.9604645e-8f;     // 2^-24
-    const float Tf = fh + fh, T2f = Tf * Tf;
-    const float e = ce + 4.4f * U * Tf;
-    const float M = ND * e * (4.f * Tf + e) + 32.f * U * T2f;
-    *lo = T2f - M;
-    *hi = T2f + M;
+    const float T2f = Tf * Tf, e = ce + 4.4f * U * Tf;
+    *T2 = T2f;
+    return ND * e * (4.f * Tf + e) + 32.f * U * T2f;
+}
+// The decision bounds of a particle's candidates, whose h lie in [h0, h1]:
+// below lo a candidate is inside the least radius, h_i + h0, and so inside its
+// own; above hi it is outside the largest; in FP64 between.  Runs with one h,
+// whatever its size, have both bounds at that radius.
+template <int ND>
+__device__ __forceinline__ void prefilter_bounds(float fh, float h0, float h1, float ce, float* lo, float* hi)
+{
+    float T2;
+    const float m0 = prefilter_margin<ND>(fh + h0, ce, &T2);
+    *lo = T2 - m0;
+    const float m1 = prefilter_margin<ND>(fh + h1, ce, &T2);
+    *hi = T2 + m1;
 }
 
 // partisearching (CPP_3-NNPS.cpp:265-374): neighbours of i in stencil order,
 // descending index inside each cell; inclusion dst <= h_i + h_j decided as the
 // reference decides it (sqrt of the FP64 sum of squares).
 //
-// Each candidate is first tested in FP32 on the (x - xmin, y - ymin, z - zmin,
-// h) records, against a margin M that bounds every rounding between the FP32
+// Each candidate is first tested in FP32 on the (x - xmin, y - ymin, z - zmin)
+// of the search's records, against a margin M that bounds every rounding between the FP32
 // squared distance d2f and the exact one: the coordinates' rounding to FP32
 // (at most 2^-24 |coordinate|, and |x_j - xmin| <= |x_i - xmin| + |x_i - x_j|),
 // the subtraction, squares and sum, and the rounding of T = h_i + h_j and T^2.
@@ -568,8 +562,8 @@ __global__ void __launch_bounds__(128, SPH_MINB_NNPS) k_nnps(Dev d)
     float Fi = fmaxf(fabsf(fx), fabsf(fy));
     if (ND == 3) Fi = fmaxf(Fi, fabsf(fz));
     float lo, hi;
-    prefilter_bounds<ND>(fh, 2.2f * U * Fi, &lo, &hi);
-    if (!(fh > 64.f * U * Fi && fh == (float)d.p.dr)) {
+    prefilter_bounds<ND>(fh, d.s.hb[0], d.s.hb[1], 2.2f * U * Fi, &lo, &hi);
+    if (!(fh > 64.f * U * Fi)) {
         // every candidate to the FP64 test
         lo = __int_as_float(0xff800000);
         hi = __int_as_float(0x7f800000);
