@@ -989,7 +989,7 @@ sphgpu_ctx* sphgpu_create(const sphgpu_params* P, int device)
     cudaEventCreate(&c->ev0);
     cudaEventCreate(&c->ev1);
     const int N = c->N;
-    const size_t M = sphk_cell_slots(P->ctotal);   // cells 0 .. ctotal, whole blocks of the scan
+    const size_t M = sphk_cell_slots(P->ctotal);   // cells 0 .. ctotal and one more, whole blocks of the scan
     Dev& d = c->d[0];
     fill_dev_params(d.p, P);
     DevState& s = d.s;

@@ -314,9 +314,8 @@ __global__ void __launch_bounds__(256) k_rain(Dev d)
 // 561-630) by counting: the particles per cell (k_cellkey), the cells' first
 // positions (k_cellsum, k_cellscan), each particle into its cell's positions in
 // any order (k_cellplace), and its rank among the cell's particles
-// (k_cellrange).  A cell holds a handful of particles, so the rank costs a few
-// broadcast loads, and the order does not depend on which particle was placed
-// first.  A radix sort of the keys moved every particle two or three times in
+// (k_cellrange), so that the order does not depend on which particle was
+// placed first.  A radix sort of the keys moved every particle two or three times in
 // six launches; with it, the cells' reset and the ranges a step of 14,978
 // particles took 0.144 ms, with these passes 0.113 (0.21 and 0.23 ms of a step
 // of 4.45 M particles).
@@ -395,29 +394,14 @@ __global__ void k_cellplace(Dev d)
     d.s.placed[q] = make_int2(i, d.s.i2o[i]);
 }
 
-// each particle's sorted position: its cell's particles in descending caller's
-// index, the order Binary_Sort's merge produces, in whatever order the state
-// is held; and the positions in that order
-__global__ void k_cellrange(Dev d)
+// particle pid, of type t at r in cell c of grid g, at sorted position q: its
+// order words and positions
+__device__ __forceinline__ void place_sorted(const Dev& d, const CellGrid& g, int c, int pid, int t, const Pos& r, int q)
 {
-    const int p = IDX, N = d.p.N;
-    if (p >= N || *d.s.err) return;
-    const int2 me = d.s.placed[p];
-    const int pid = me.x, c = d.s.cell[pid], first = d.s.cofs[c];
-    // positions of the same cell on both sides of p
-    int q = first;
-    for (int r = first; r < N; r++) {
-        const int2 o = d.s.placed[r];
-        if (r > p && d.s.cell[o.x] != c) break;
-        q += o.y > me.y;
-    }
-    const CellGrid g = cell_grid(d, pid);
     d.s.pid_sorted[q] = pid;
     d.s.ckey[q] = c;
     d.s.sortpos[pid] = q;
-    const int t = d.s.type[pid];
     const int w = (pid << 3) | ((t >= 0 && t <= 4) ? t : 7);
-    const Pos r = load_pos(d.s.xh, pid);
     store_pos(d.s.xs, q, r);
     // the search's FP32 records with the index-and-type word, and its planes;
     // a candidate whose h lies outside the context's bounds (or is not a
@@ -426,10 +410,136 @@ __global__ void k_cellrange(Dev d)
     const float hj = (float)r.h;
     if (!(hj >= d.s.hb[0] && hj <= d.s.hb[1])) f.x = __int_as_float(0x7fffffff);
     reinterpret_cast<float4*>(d.s.xsf)[q] = f;
-    const size_t NP = (size_t)SPH_XSP_STRIDE(N);
+    const size_t NP = (size_t)SPH_XSP_STRIDE(d.p.N);
     d.s.xsp[q] = f.x;
     d.s.xsp[NP + q] = f.y;
     d.s.xsp[2 * NP + q] = f.z;
+}
+
+// A crowded cell's n particles, at positions first .. first + n - 1 in any
+// order, into descending caller's index, by one block of 256 threads: a radix
+// sort of the reversed indices, eight bits a pass, stable, 1,024 particles at a
+// time: a warp takes 128 consecutive ones, 32 by 32, each one's rank among
+// the equal digits of its warp by a match and the warp's count so far.  The
+// passes go from `placed` to two scratch arrays in turn, both in the
+// provisional lists, which the search has yet to write.
+__device__ __noinline__ void sort_crowded(const Dev& d, int c, int first, int n)
+{
+    constexpr int T = 256, W = T / 32, U = 4;
+    __shared__ int base[T], at[W][T];
+    typedef cub::BlockScan<int, T> Scan;
+    __shared__ typename Scan::TempStorage tmp;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, N = d.p.N;
+    int2* buf[2] = {reinterpret_cast<int2*>(d.s.nbrs) + first, reinterpret_cast<int2*>(d.s.nbrs) + (size_t)N + first};
+    const int2* src = d.s.placed + first;
+    int turn = 0;
+    for (int shift = 0; shift == 0 || ((N - 1) >> shift) != 0; shift += 8, turn ^= 1) {
+        int2* dst = buf[turn];
+        base[t] = 0;
+        for (int w = 0; w < W; w++) at[w][t] = 0;
+        __syncthreads();
+        for (int e0 = 0; e0 < n; e0 += U * T) {
+            int y[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) y[u] = (e0 + u * T + t < n) ? src[e0 + u * T + t].y : -1;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int dg = (y[u] >= 0) ? ((N - 1 - y[u]) >> shift) & 0xff : -1;
+                const unsigned same = __match_any_sync(0xffffffffu, dg);
+                if (y[u] >= 0 && (same & ((1u << lane) - 1u)) == 0u) atomicAdd(&base[dg], __popc(same));
+            }
+        }
+        __syncthreads();
+        int from;
+        Scan(tmp).ExclusiveSum(base[t], from);
+        base[t] = from;
+        for (int e0 = 0; e0 < n; e0 += U * T) {
+            int2 v[U];
+            int rank[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int e = e0 + warp * 32 * U + 32 * u + lane;
+                v[u] = (e < n) ? src[e] : make_int2(0, -1);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const bool in = v[u].y >= 0;
+                const int dg = in ? ((N - 1 - v[u].y) >> shift) & 0xff : -1;
+                const unsigned same = __match_any_sync(0xffffffffu, dg);
+                const int r = __popc(same & ((1u << lane) - 1u)), before = in ? at[warp][dg] : 0;
+                __syncwarp();
+                if (in && r == 0) at[warp][dg] = before + __popc(same);
+                __syncwarp();
+                rank[u] = before + r;
+            }
+            __syncthreads();
+            int o = base[t];                     // this thread's digit: where each warp's go
+            for (int w = 0; w < W; w++) {
+                const int k = at[w][t];
+                at[w][t] = o;
+                o += k;
+            }
+            base[t] = o;
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (v[u].y >= 0) dst[at[warp][((N - 1 - v[u].y) >> shift) & 0xff] + rank[u]] = v[u];
+            __syncthreads();
+            for (int w = 0; w < W; w++) at[w][t] = 0;
+            __syncthreads();
+        }
+        src = dst;
+    }
+    const CellGrid g = cell_grid(d, src[0].x);       // a cell belongs to one grid
+    for (int e0 = t; e0 < n; e0 += U * T) {
+        int pid[U], ty[U];
+        Pos r[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) pid[u] = src[min(e0 + u * T, n - 1)].x;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            ty[u] = d.s.type[pid[u]];
+            r[u] = load_pos(d.s.xh, pid[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (e0 + u * T < n) place_sorted(d, g, c, pid[u], ty[u], r[u], first + e0 + u * T);
+    }
+}
+
+// Each particle's sorted position: its cell's particles in descending caller's
+// index, the order Binary_Sort's merge produces, in whatever order the state
+// is held; and the positions in that order.  A particle counts the later ones
+// of its cell, one load each: a cell at the spacing holds a handful (lattice
+// 8 per phase).  Cells of more than SPH_CROWDED particles (water that left the
+// box is parked past its ends and is never searched, so nothing bounds their
+// number) are sorted by the block that holds their first position, at most
+// one per block: 100,000 and 400,000 particles in one cell take 1.2 and 4.8
+// ms; counting alone took 12.7 and 117.  At 32 registers, as without the sort:
+// with the 78 it takes unbounded, fewer blocks hide the ordinary cells' loads.
+#define SPH_CROWDED 512
+__global__ void __launch_bounds__(256, 8) k_cellrange(const __grid_constant__ Dev d)
+{
+    static_assert(SPH_CROWDED >= 256, "one crowded cell per block");
+    const int p = IDX, N = d.p.N;
+    if (*d.s.err) return;
+    __shared__ int crowded[3];
+    bool mine = false;
+    if (p < N) {
+        const int2 me = d.s.placed[p];
+        const int c = d.s.cell[me.x], first = d.s.cofs[c], n = d.s.cofs[c + 1] - first;
+        if (n <= SPH_CROWDED) {
+            int q = first;
+            for (int r = first; r < first + n; r++) q += d.s.placed[r].y > me.y;
+            place_sorted(d, cell_grid(d, me.x), c, me.x, d.s.type[me.x], load_pos(d.s.xh, me.x), q);
+        } else if (p == first) {
+            mine = true;
+            crowded[0] = c;
+            crowded[1] = first;
+            crowded[2] = n;
+        }
+    }
+    if (__syncthreads_or(mine)) sort_crowded(d, crowded[0], crowded[1], crowded[2]);
 }
 
 // The FP64 inclusion test of one candidate, as partisearching decides it:
@@ -3310,10 +3420,11 @@ __global__ void k_check_lists(Dev d)
 }
 #endif
 
-// the cells the counts are kept for: whole blocks of the scan
+// the cells the counts are kept for: 0 .. ctotal and one more, whose first
+// position is where the last one's end, in whole blocks of the scan
 extern "C" size_t sphk_cell_slots(int ctotal)
 {
-    return ((size_t)ctotal + 1 + SPH_SCAN_CELLS - 1) / SPH_SCAN_CELLS * SPH_SCAN_CELLS;
+    return ((size_t)ctotal + 2 + SPH_SCAN_CELLS - 1) / SPH_SCAN_CELLS * SPH_SCAN_CELLS;
 }
 
 extern "C" int sphk_enqueue_nnps_parts(const Dev* dp, cudaStream_t st, cudaEvent_t* ev, int parts)
