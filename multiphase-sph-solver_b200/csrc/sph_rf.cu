@@ -107,10 +107,12 @@ __global__ void k_rf_corr(RFArgs a, double* C)
 // latency: 64 steps of a reciprocal root and two barriers, then 64 of a
 // broadcast and a quotient: 36 us a panel (45 with a square root and a
 // reciprocal each; 130 with one thread per row).
+// (An infinite x, as rotated kernels of short correlation lengths give, leaves
+// no finite residual: its quotient is the product.)
 __device__ __forceinline__ double rf_quotient(double x, double y, double ry)
 {
-    const double q = x * ry;
-    return fma(fma(-q, y, x), ry, q);
+    const double q = x * ry, r = fma(-q, y, x);
+    return isfinite(r) ? fma(r, ry, q) : q;
 }
 
 __global__ void __launch_bounds__(4 * RF_B) k_rf_panel(double* A, double* diag, int n, int k0)
