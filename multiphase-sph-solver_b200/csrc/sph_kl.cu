@@ -187,7 +187,10 @@ extern "C" int sphk_kl_field(int n, int ndim, int K, int no, int type, const dou
         nm += a.nmode[d];
     }
     auto launch = [&](auto kernel, int threads, size_t smem) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 1;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            cudaGetLastError();     // refused: not left for a later call's check
+            return 1;
+        }
         kernel<<<(unsigned)((n + threads - 1) / threads), threads, smem, st>>>(a);
         return cudaGetLastError() == cudaSuccess ? 0 : 1;
     };

@@ -336,7 +336,10 @@ extern "C" int sphk_rf_factor(const int* ip, const double* dp, double* d_C, cuda
     k_rf_corr<<<dim3((T + 255) / 256, T), 256, 0, st>>>(a, d_C);
     double* d_diag = d_C + (size_t)T * T;
     const int smem = 2 * RF_B * RF_LD * (int)sizeof(double);
-    if (cudaFuncSetAttribute(k_rf_update, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 1;
+    if (cudaFuncSetAttribute(k_rf_update, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
     for (int k0 = 0; k0 < T; k0 += RF_B) {
         const int rest = T - k0 - RF_B;
         const int tiles = (rest > 0) ? (rest + RF_B - 1) / RF_B : 0;
