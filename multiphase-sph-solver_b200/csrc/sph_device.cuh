@@ -498,15 +498,26 @@ __device__ __forceinline__ double div_rcp_fast(double x, double y, double yr, bo
 }
 
 // v[k] / y for each k, y's correctly rounded reciprocal yr at hand (FP64); one
-// test for all of them in place of a division's slow path each.  The FP32
-// form divides.
+// test for all of them in place of a division's slow path each.  These
+// numerators reach the bottom of the range (velocity differences ahead of a
+// disturbance), where the residual is rounded and the correction with it: a
+// residual that is not finite, subnormal or zero sends all of the pair's to
+// the IEEE division unless its numerator is zero (whose quotient is the
+// product, sign included).  The FP32 form divides.
 template <int K>
 __device__ __forceinline__ void quotients(double (&v)[K], double y, double yr)
 {
-    bool bad = false;
+    bool bad = (__double2hiint(yr) & 0x7ff00000) == 0x7ff00000;       // y is zero, subnormal or not a number
     double q[K];
 #pragma unroll
-    for (int k = 0; k < K; k++) q[k] = div_rcp_fast(v[k], y, yr, bad);
+    for (int k = 0; k < K; k++) {
+        const double p = __dmul_rn(v[k], yr);
+        const double r = __fma_rn(-p, y, v[k]);
+        // the exponent 0 or all ones (the sum then carries into the sign)
+        const bool special = ((__double2hiint(r) + 0x00100000) & 0x7fe00000) == 0, some = v[k] != 0.0;
+        q[k] = some ? __fma_rn(r, yr, p) : p;
+        bad |= special && some;
+    }
     if (bad) {
 #pragma unroll
         for (int k = 0; k < K; k++) q[k] = v[k] / y;
