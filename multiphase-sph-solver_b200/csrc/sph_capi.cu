@@ -186,9 +186,10 @@ struct sphgpu_ctx {
     std::condition_variable out_cv;
     long out_ticket = 0, out_turn = 0;
     // device scratch of the random-field calls, kept from one to the next
-    // while it is small (field_scratch)
+    // while it is small (FieldScratch), and whether a call is using it
     void* fs[3] = {nullptr, nullptr, nullptr};
     size_t fs_bytes[3] = {0, 0, 0};
+    bool fs_used[3] = {false, false, false};
     std::vector<InstGrid> h_inst;     // batched context: the instance table (empty: one system)
     InstGrid* d_inst = nullptr;
     // the re-sorted state (sphgpu_set_reorder): re-sort every reorder_every
@@ -676,6 +677,17 @@ void* field_ptr(sphgpu_ctx* c, const char* name)
     for (auto& t : tab)
         if (std::strcmp(t.n, name) == 0) return t.p;
     return nullptr;
+}
+
+// the random-field scratch that no call is using, given back
+void release_field_scratch(sphgpu_ctx* c)
+{
+    for (int k = 0; k < 3; k++)
+        if (c->fs[k] && !c->fs_used[k]) {
+            cudaFree(c->fs[k]);
+            c->fs[k] = nullptr;
+            c->fs_bytes[k] = 0;
+        }
 }
 
 // whether the strain pass takes the artificial-viscosity sums in the steps to
@@ -1609,6 +1621,7 @@ int run_parts(sphgpu_ctx* c, int upto)
         if (r) return r;
     }
     cudaSetDevice(c->device);
+    release_field_scratch(c);
     if (c->part_done == 0) {
         // the method entries run on the caller's order
         int r = to_caller_order(c);
@@ -1781,6 +1794,7 @@ int sphgpu_step(sphgpu_ctx* c, int nsteps)
         for (long long l = c->l_host; l < (long long)c->l_host + nsteps; l++)
             if (l % c->P.step_regu == 0) { c->regu = true; invalidate_graphs(c); break; }
     cudaSetDevice(c->device);
+    release_field_scratch(c);
     set_visc(c);
     if (!c->exec[0] || !c->exec[1]) {
         r = build_graphs(c);
@@ -2466,6 +2480,7 @@ int sphgpu_step_profiled(sphgpu_ctx* c, int nsteps, double* stage_ms)
         for (long long l = c->l_host; l < (long long)c->l_host + nsteps; l++)
             if (l % c->P.step_regu == 0) { c->regu = true; invalidate_graphs(c); break; }
     cudaSetDevice(c->device);
+    release_field_scratch(c);
     cudaEvent_t ev[SPHK_NSTAGES + 1];
     for (int k = 0; k <= SPHK_NSTAGES; k++) CK(cudaEventCreate(&ev[k]));
     for (int k = 0; k < SPHK_NSTAGES; k++) stage_ms[k] = 0.0;
@@ -2716,11 +2731,12 @@ void kl_solve_wi(std::vector<double>& wi, const double a_x[3], const double rl[3
 
 struct HostKLTerm { double w, alpha; int use_cos; int pad; };
 
-// Device scratch of one random-field call, given back at its end.  Buffers of
-// up to 256 MB stay with the context for the next call (allocating and freeing
-// 190 MB took 2 of the 10 ms of a correlation-matrix field's call); larger ones
-// are freed.  Slots: 0 a plan's or field's small arrays, 1 the field's values, 2 the
-// correlation matrix and its vectors.
+// Device scratch of one random-field call.  Buffers of up to 256 MB stay with
+// the context for the next field (allocating and freeing 190 MB took 2 of the 10
+// ms of a correlation-matrix field's call) until it steps again, or another
+// field's buffer finds no room (release_field_scratch); larger ones are freed
+// with the call.  Slots: 0 a plan's or field's small arrays, 1 the field's
+// values, 2 the correlation matrix and its vectors.
 struct FieldScratch {
     sphgpu_ctx* c;
     int slot;
@@ -2733,14 +2749,23 @@ struct FieldScratch {
             if (c->fs[slot]) cudaFree(c->fs[slot]);
             c->fs[slot] = nullptr;
             c->fs_bytes[slot] = 0;
-            CK(cudaMalloc(&c->fs[slot], bytes));
+            cudaError_t e = cudaMalloc(&c->fs[slot], bytes);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                release_field_scratch(c);
+                e = cudaMalloc(&c->fs[slot], bytes);
+            }
+            if (e != cudaSuccess) c->fs[slot] = nullptr;
+            CK(e);
             c->fs_bytes[slot] = bytes;
         }
+        c->fs_used[slot] = true;
         p = static_cast<char*>(c->fs[slot]);
         return 0;
     }
     ~FieldScratch()
     {
+        c->fs_used[slot] = false;
         if (c->fs_bytes[slot] > ((size_t)256 << 20)) {
             cudaFree(c->fs[slot]);
             c->fs[slot] = nullptr;
