@@ -426,10 +426,11 @@ long   sphgpu_last_step_launches(const sphgpu_ctx* ctx);
  * each pass the fastest, a shape other than 128 only when it is more than 3%
  * faster (the spread of the timings).  The steps it runs are steps of the
  * run: a launch shape changes no result, bit for bit.  With cache_path the
- * choice is kept in that text file under a key of the GPU model and the
- * run's shape (dimension, particle count, wall, drag and contact types,
- * precision form, instances), and a later call with the same key applies it
- * without measuring.  table, if non-NULL, receives the mean ms per step of
+ * choice is kept in that text file under a key of the passes' version, the GPU
+ * model and the run's shape (dimension, particle count, wall, drag, contact
+ * and vibration types, before or past the damped steps, precision form,
+ * instances), and a later call with the same key applies it without
+ * measuring.  table, if non-NULL, receives the mean ms per step of
  * each pass for each candidate (4 x SPHGPU_TUNE_PASSES, candidate-major).
  */
 #define SPHGPU_TUNE_PASSES 10

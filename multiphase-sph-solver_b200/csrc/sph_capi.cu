@@ -2544,7 +2544,10 @@ void set_tb(sphgpu_ctx* c, const int* tb)
     invalidate_graphs(c);
 }
 
-// what a tuned shape is kept for: the GPU model and the run's shape
+// what a tuned shape is kept for: the passes as this build has them (a number
+// that changes with them), the GPU model, the run's shape and what chooses the
+// passes' variants
+constexpr int kTuneKernels = 2;
 std::string tune_key(const sphgpu_ctx* c)
 {
     cudaDeviceProp prop;
@@ -2553,8 +2556,9 @@ std::string tune_key(const sphgpu_ctx* c)
     for (char& ch : name)
         if (ch == ' ') ch = '_';
     char buf[256];
-    std::snprintf(buf, sizeof(buf), "%s/ndim%d/n%d/flbndy%d/fli%d/ss%d/prec%d/inst%d", name.c_str(), c->P.ndim,
-                  c->N, c->P.flbndy, c->P.fli, c->P.ss_type, c->precision, (int)c->h_inst.size());
+    std::snprintf(buf, sizeof(buf), "%s/k%d/ndim%d/n%d/flbndy%d/fli%d/ss%d/flv%d/visc%d/prec%d/inst%d", name.c_str(),
+                  kTuneKernels, c->P.ndim, c->N, c->P.flbndy, c->P.fli, c->P.ss_type, c->P.flv, c->d[0].p.visc,
+                  c->precision, (int)c->h_inst.size());
     return buf;
 }
 
@@ -2579,6 +2583,7 @@ int sphgpu_get_launch(const sphgpu_ctx* c, int* tb, int n)
 int sphgpu_autotune(sphgpu_ctx* c, int steps, const char* cache_path, double* table)
 {
     if (!c || steps <= 0) return SPHGPU_E_ARG;
+    set_visc(c);
     const std::string key = tune_key(c);
     if (cache_path) {
         if (FILE* f = std::fopen(cache_path, "r")) {
@@ -2626,7 +2631,8 @@ int sphgpu_autotune(sphgpu_ctx* c, int steps, const char* cache_path, double* ta
         best[q] = cand[b];
     }
     set_tb(c, best);
-    if (cache_path) {
+    // (not kept where the passes changed while they were timed)
+    if (cache_path && tune_key(c) == key) {
         if (FILE* f = std::fopen(cache_path, "a")) {
             std::fprintf(f, "%s", key.c_str());
             for (int q = 0; q < TP_COUNT; q++) std::fprintf(f, " %d", best[q]);
