@@ -419,7 +419,9 @@ long   sphgpu_last_step_launches(const sphgpu_ctx* ctx);
  * SPHGPU_TUNE_PASSES neighbour passes -- the search scan, its resolve pass,
  * the pair records, density, Shepard + EOS, strain, the constitutive update,
  * the two momentum stages, XSPH + update, in that order -- runs one particle
- * per thread with 32 to 128 threads per block (a multiple of 32).
+ * per thread with 32 to 128 threads per block (a multiple of 32).  The resolve
+ * pass is part of the pair records: its entry is kept for the arrays' layout
+ * and has no effect, and the autotuner repeats theirs there.
  * sphgpu_set_launch / sphgpu_get_launch set and read those sizes;
  * sphgpu_autotune runs `steps` steps of the run with each of 32, 64, 96 and
  * 128 threads per block, times every pass with CUDA events, and keeps for

@@ -2525,7 +2525,7 @@ static_assert(TP_COUNT == SPHGPU_TUNE_PASSES, "tuned passes");
 
 // the stages (sphk_stage_names) whose device time each tuned pass is
 const char* const kTuneStages[TP_COUNT][2] = {
-    {"k_nnps", nullptr}, {"k_nnps_resolve", nullptr}, {"k_pairw", nullptr}, {"k_density", nullptr},
+    {"k_nnps", nullptr}, {"k_pairw", nullptr}, {"k_pairw", nullptr}, {"k_density", nullptr},
     {"k_shepard_eos", nullptr}, {"k_strain", nullptr}, {"k_stress", "k_stress_2"}, {"k_accel_a", nullptr},
     {"k_accel_b", nullptr}, {"k_xsph_update", nullptr},
 };

@@ -43,7 +43,7 @@
 #define SPH_SCAN_CELLS 1024    // cells per block of the cell scan: 4 per thread
 #define SPH_ERR_CELL 3         // parttocell, CPP_3-NNPS.cpp:247-257
 #define SPH_ERR_NEIGH 5        // partisearching, CPP_3-NNPS.cpp:313-319
-#define SPHK_NSTAGES 21        // entries of sphk_stage_names (one event bracket each)
+#define SPHK_NSTAGES 20        // entries of sphk_stage_names (one event bracket each)
 #ifndef SPHGPU_CHECK
 #define SPHGPU_CHECK 0         // 1: the bounds-checked build (k_check_lists after the search)
 #endif
@@ -62,7 +62,9 @@ struct InstGrid {
 
 // Passes whose threads per block the autotuner picks (one particle per
 // thread; every pass is written for any multiple of 32 up to its launch
-// bound of 128)
+// bound of 128).  TP_RESOLVE launches nothing: the resolve pass of the search is
+// part of the pair-record pass, whose choice its entry follows; the launch
+// arrays of the C ABI keep its place.
 enum TunePass {
     TP_NNPS, TP_RESOLVE, TP_PAIRW, TP_DENSITY, TP_SHEPARD, TP_STRAIN, TP_STRESS, TP_ACCEL_A, TP_ACCEL_B,
     TP_XSPH, TP_COUNT

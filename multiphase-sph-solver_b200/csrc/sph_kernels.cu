@@ -3368,7 +3368,7 @@ extern "C" int sphk_order_sort(const Dev* dp, void* tmp, size_t bytes, int end_b
 // before stage k and ev[SPHK_NSTAGES] after the last one (stages a run does
 // not need are recorded with no work between their events).
 extern "C" const char* const sphk_stage_names[] = {
-    "k_cellkey", "k_cellscan", "k_cellplace", "k_cellrange", "k_nnps", "k_nnps_resolve", "k_pairw", "k_kgc",
+    "k_cellkey", "k_cellscan", "k_cellplace", "k_cellrange", "k_nnps", "k_pairw", "k_kgc",
     "k_density", "k_shepard_eos", "k_strain", "k_regu_eps", "k_stress", "k_regu_sig", "k_stress_2",
     "k_art_rij", "k_accel_a", "k_accel_b", "k_xsph_update", "k_tm_boundary", "k_step_done"};
 static_assert(sizeof(sphk_stage_names) / sizeof(sphk_stage_names[0]) == SPHK_NSTAGES, "stage table");
@@ -3449,14 +3449,13 @@ extern "C" int sphk_enqueue_nnps_parts(const Dev* dp, cudaStream_t st, cudaEvent
         REC(4);
         LAUNCH_ND(k_nnps, nblk(N, tbk(d, TP_NNPS)), tbk(d, TP_NNPS), d); n++;
         REC(5);
-        REC(6);
         LAUNCH_ND(k_pairw, nblk(N, tbk(d, TP_PAIRW)), tbk(d, TP_PAIRW), d); n++;
 #if SPHGPU_CHECK
         k_check_lists<<<nblk(N, 128), 128, 0, st>>>(d); n++;
 #endif
     }
     if (parts & 4) {
-        REC(7);
+        REC(6);
         if (d.p.flknl > 2) { LAUNCH_ND(k_kgc, nblk(N, 128), 128, d); n++; }
     }
     return n;
@@ -3477,11 +3476,11 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
     d.s.eps_in = regu ? d.s.eps_tmp : d.s.eps;
     const int N = d.p.N;
     int n = 0;
-    REC(8);
+    REC(7);
     LAUNCH_ND(k_density, nblk(N, tbk(d, TP_DENSITY)), tbk(d, TP_DENSITY), d); n++;
-    REC(9);
+    REC(8);
     LAUNCH_ND(k_shepard_eos, nblk(N, tbk(d, TP_SHEPARD)), tbk(d, TP_SHEPARD), d); n++;
-    REC(10);
+    REC(9);
     const bool visc = sizeof(real) == 8 && d.p.visc;
     {
         const unsigned tb = tbk(d, TP_STRAIN), g = nblk(N, tb);
@@ -3495,9 +3494,9 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
         n++;
     }
     if (d.p.flagum == 1) { k_saturation<<<nblk(N, 128), 128, 0, st>>>(d); n++; }
-    REC(11);
+    REC(10);
     if (regu) { LAUNCH_ND(k_regu, nblk(N, 128), 128, d, d.s.eps, d.s.eps_tmp, 1); n++; }
-    REC(12);
+    REC(11);
     const unsigned sb = tbk(d, TP_STRESS), sg = nblk(N, sb);
     auto stress = [&](auto phase) {
         constexpr int PH = decltype(phase)::value;
@@ -3518,14 +3517,14 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
     };
     if (regu) stress(std::integral_constant<int, 1>());
     else stress(std::integral_constant<int, 0>());
-    REC(13);
+    REC(12);
     if (regu) { LAUNCH_ND(k_regu, nblk(N, 128), 128, d, d.s.sig_next, d.s.sig_tmp, 0); n++; }
-    REC(14);
+    REC(13);
     if (regu) stress(std::integral_constant<int, 2>());
-    REC(15);
+    REC(14);
     const bool art = d.p.art_stre_coe > 0.0;
     if (art) { LAUNCH_ND(k_art_rij, nblk(N, 128), 128, d); n++; }
-    REC(16);
+    REC(15);
     LAUNCH_ND(k_accel_a, nblk(N, tbk(d, TP_ACCEL_A)), tbk(d, TP_ACCEL_A), d); n++;
     if (d.p.flbndy == 5) { LAUNCH_ND(k_free_solid, nblk(N, 128), 128, d); n++; }
     if (d.p.ss_coupled) { LAUNCH_ND(k_coupled, nblk(N, 128), 128, d); n++; }
@@ -3533,7 +3532,7 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
         LAUNCH_ND(k_ss_pair, nblk(N, 128), 128, d); n++;
         k_ss_struct<<<nblk(N, 128), 128, 0, st>>>(d); n++;
     }
-    REC(17);
+    REC(16);
     {
         const bool drag = d.p.fli > 1, vib = d.p.flv != 0;
         const dim3 g(nblk(N, tbk(d, TP_ACCEL_B))), b(tbk(d, TP_ACCEL_B));
@@ -3578,9 +3577,9 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
         }
         n++;
     }
-    REC(18);
+    REC(17);
     LAUNCH_ND(k_xsph_update, nblk(N, tbk(d, TP_XSPH)), tbk(d, TP_XSPH), d); n++;
-    REC(19);
+    REC(18);
     if (d.p.flbndy == 2) {
         LAUNCH_ND(k_tm_vb, nblk(N, 128), 128, d); n++;
         k_tm_wall<<<nblk(N, 128), 128, 0, st>>>(d); n++;
@@ -3589,8 +3588,8 @@ extern "C" int SPHK_ENTRY(sphk_enqueue_physics)(const Dev* dp, cudaStream_t st, 
     }
     if (d.p.flr) { k_partidel<<<nblk(N, 256), 256, 0, st>>>(d); n++; }
     if (d.p.cfl_on) { k_cfl<<<148 * 8, 256, 0, st>>>(d); n++; }
-    REC(20);
+    REC(19);
     k_step_done<<<1, 32, 0, st>>>(d); n++;
-    REC(21);
+    REC(20);
     return n;
 }

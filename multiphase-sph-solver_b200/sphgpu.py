@@ -527,6 +527,7 @@ class Engine:
     def update(self) -> int:
         return int(self.lib.sphgpu_update(self.h))
 
+    # (k_nnps_resolve is part of k_pairw: its entry has no effect)
     TUNE_PASSES = ("k_nnps", "k_nnps_resolve", "k_pairw", "k_density", "k_shepard_eos", "k_strain", "k_stress",
                    "k_accel_a", "k_accel_b", "k_xsph_update")
 

@@ -54,3 +54,14 @@ def test_lines_of_other_passes_are_not_applied(tmp_path):
     assert (eng.autotune(1, str(cache)) > 0).any()
     assert len(_lines(cache)) == 2
     eng.close()
+
+
+def test_every_stage_is_a_pass():
+    """The resolve pass is part of the pair records: no stage of its own, and
+    its entry of the launch shape follows theirs."""
+    eng = _engine()
+    assert "k_nnps_resolve" not in eng.step_profiled(1)
+    table, chosen = eng.autotune(1), eng.launch()
+    resolve, pairw = (eng.TUNE_PASSES.index(k) for k in ("k_nnps_resolve", "k_pairw"))
+    assert np.array_equal(table[:, resolve], table[:, pairw]) and chosen[resolve] == chosen[pairw]
+    eng.close()
