@@ -124,6 +124,18 @@ def fp64_roofline(device: int, n: int, step_ms: float) -> dict:
             "fp32_peak": f32}
 
 
+# The kernels of a stage as ncu_traffic names them, where a stage launches
+# others than the one it is named for: past the damped steps the momentum stage
+# is the drag loop and the tail kernel (the viscosity sums are the strain
+# pass's).
+STAGE_KERNELS = {"k_accel_b": ("k_accel_b_drag", "k_accel_b_tail")}
+
+
+def traffic_kernels(stages, stage_ms: dict) -> list:
+    """The kernels that the stages launched, of those that ran."""
+    return [q for k in stages if stage_ms.get(k, 0.0) > 0.01 for q in STAGE_KERNELS.get(k, (k,))]
+
+
 def measured_peaks() -> tuple[dict, str]:
     p = os.path.join(REPO, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -682,10 +694,7 @@ def engine_arm(args, world, rank, local):
     avg_ms = dom["ms"]
     alg = dom["bytes_per_particle"] * scene.n
     achieved = dom["achieved_gbs"]
-    # the pass's kernels as ncu names them (the momentum stage launches two
-    # loop kernels and a tail kernel under the stage name k_accel_b)
-    ncu_names = {"k_accel_b": ("k_accel_b", "k_accel_b_drag", "k_accel_b_tail")}
-    pass_kernels = [q for k in dom["kernels"] if stage_ms.get(k, 0.0) > 0.01 for q in ncu_names.get(k, (k,))]
+    pass_kernels = traffic_kernels(dom["kernels"], stage_ms)
     per_kernel = ncu_traffic()
     traffic = (sum(per_kernel[k] for k in pass_kernels)
                if pass_kernels and all(k in per_kernel for k in pass_kernels) else None)
