@@ -60,7 +60,7 @@ WORKLOAD = "3d_saturated_soil_column_collapse"
 RESORT_EVERY = 20
 PASS_BYTES_2D = {
     "key": 24.0,
-    "radix sort": 32.0,
+    "cell sort": 32.0,
     "reorder": 196.0,
     "cell ranges": 14.0,
     "porosity + continuity": 68.0,
@@ -72,7 +72,7 @@ PASS_BYTES_2D = {
 STEP_BYTES_3D = 1870.0
 PASS_KERNELS = {
     "key": ("k_cellkey",),
-    "radix sort": ("k_cellscan", "k_cellplace"),
+    "cell sort": ("k_cellscan", "k_cellplace"),
     "reorder": ("reorder",),
     "cell ranges": ("k_cellrange",),
     "porosity + continuity": ("k_density",),
@@ -134,6 +134,25 @@ STAGE_KERNELS = {"k_accel_b": ("k_accel_b_drag", "k_accel_b_tail")}
 def traffic_kernels(stages, stage_ms: dict) -> list:
     """The kernels that the stages launched, of those that ran."""
     return [q for k in stages if stage_ms.get(k, 0.0) > 0.01 for q in STAGE_KERNELS.get(k, (k,))]
+
+
+def download_record_bytes() -> int:
+    """Bytes per particle of sphgpu_download_particles: the device-owned
+    members (all but x) as they lie in a packed record, doubles at multiples of
+    8 bytes and ints in 4, the record a multiple of 8."""
+    import ctypes
+
+    import sphgpu
+    lib = sphgpu.load_library()
+    members = []
+    for name in sphgpu.FIELDS:
+        off, nc = ctypes.c_size_t(0), ctypes.c_int(0)
+        if name != "x" and lib.sphgpu_particle_layout(name.encode(), ctypes.byref(off), ctypes.byref(nc)) == 0:
+            members.append((off.value, nc.value, name in sphgpu.INT_FIELDS))
+    size = 0
+    for _, nc, is_int in sorted(members):
+        size = size + 4 * nc if is_int else -(-size // 8) * 8 + 8 * nc
+    return -(-size // 8) * 8
 
 
 def measured_peaks() -> tuple[dict, str]:
@@ -717,9 +736,7 @@ def engine_arm(args, world, rank, local):
     t_e2e = time.perf_counter() - t0
     t_e2e = dist_max(t_e2e, world)
     h2d = recs.nbytes + fluid.nbytes + soil.nbytes
-    # the download moves the device-owned members only (all but x), ints in
-    # 8-byte slots
-    d2h = scene.n * sum(8 * nc if k not in sphgpu.INT_FIELDS else 8 for k, nc in sphgpu.FIELDS.items() if k != "x")
+    d2h = scene.n * download_record_bytes()
     e2e_value = total_active * args.steps / t_e2e
     eng2.close()
 

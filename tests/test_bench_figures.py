@@ -1,5 +1,6 @@
 """bench.py's own figures on the CPU: the kernels whose traffic it adds up are
-the ones the step launches, and the committed traffic names them all."""
+the ones the step launches, the committed traffic names them all, and the
+download's bytes are those of the packed records."""
 import os
 import sys
 
@@ -31,3 +32,8 @@ def test_committed_traffic_covers_the_heavy_passes():
             assert per_kernel[k] > 0.0, k
     # kernels that are no longer launched
     assert not {"k_nnps_resolve", "k_accel_b"} & set(per_kernel)
+
+
+def test_download_bytes_are_the_packed_records():
+    # 73 doubles and four ints of Particle, without x
+    assert bench.download_record_bytes() == 73 * 8 + 4 * 4
