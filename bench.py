@@ -728,13 +728,13 @@ def engine_arm(args, world, rank, local):
     fluid, soil = np.ascontiguousarray(st.fluid), np.ascontiguousarray(st.soil)
     eng2 = sphgpu.Engine(st.params, device=local if world > 1 else args.device)
     barrier(world)
-    t0 = time.perf_counter()
-    eng2.upload_particles(recs)
-    eng2.set_materials(fluid, soil)
-    eng2.step(args.steps)
-    eng2.download_particles(out_recs)
-    t_e2e = time.perf_counter() - t0
-    t_e2e = dist_max(t_e2e, world)
+    marks = [time.perf_counter()]
+    for call in (lambda: eng2.upload_particles(recs), lambda: eng2.set_materials(fluid, soil),
+                 lambda: eng2.step(args.steps), lambda: eng2.download_particles(out_recs)):
+        call()
+        marks.append(time.perf_counter())
+    e2e_s = dict(zip(("upload", "materials", "steps", "download"), (b - a for a, b in zip(marks, marks[1:]))))
+    t_e2e = dist_max(marks[-1] - marks[0], world)
     h2d = recs.nbytes + fluid.nbytes + soil.nbytes
     d2h = scene.n * download_record_bytes()
     e2e_value = total_active * args.steps / t_e2e
@@ -845,6 +845,7 @@ def engine_arm(args, world, rank, local):
             "rf_cholesky": rf,
             "e2e": {"value": e2e_value, "unit": "particle-updates/s",
                     "h2d_bytes_per_step": h2d / args.steps, "d2h_bytes_per_step": d2h / args.steps,
+                    "seconds": e2e_s,
                     "what": "Particle-record upload, material upload, K steps and Particle-record download "
                             "through the C ABI"},
             "cpu_baseline": cpu,
