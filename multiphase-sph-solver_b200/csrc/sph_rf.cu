@@ -15,7 +15,7 @@
 //   k_rf_panel   a 64-column panel: its diagonal block factored, the rows below
 //                solved against it
 //   k_rf_update  the trailing lower triangle less the panel's outer product
-//                (64 x 64 output tiles, FP64 tensor-core products)
+//                (64 x 64 output tiles)
 //   k_rf_gemv    E = L zeta, one warp per row
 //   k_rf_assign  each particle's value from its cell (normal or lognormal map
 //                with the depth trend, as the reference writes it)
@@ -176,17 +176,17 @@ __global__ void __launch_bounds__(4 * RF_B) k_rf_panel(double* A, double* diag, 
 }
 
 // the trailing lower triangle, A[i][j] -= sum_k L[i][k] L[j][k] over the
-// panel's 64 columns, for k0 + 64 <= j <= i < n: 64 x 64 output tiles, both
-// operands' panels staged whole in shared memory, the products on the FP64
-// tensor cores (mma.sync m8n8k4, the tensor form that takes FP64): eight warps
-// of 16 x 32 outputs, 2 x 4 products per four columns from six operand loads.
-// Rows are padded to 68 doubles: the four columns of eight rows then fall in
-// distinct banks.  Three blocks per SM (80 registers, a few spills): with two
-// the outputs' loads are not hidden.  One update of 4,766 rows: 20 us; 38 us
-// with multiply-adds on an 8 x 4 register block.  Whole call, 4,830 cells 20.0 ->
-// 7.8 ms, 13,230 cells 83 -> 68 ms, the error against 64 bits unchanged.
-#define RF_LD 68
-__global__ void __launch_bounds__(256, 3) k_rf_update(double* A, const double* diag, int n, int k0)
+// panel's 64 columns, for k0 + 64 <= j <= i < n: 64 x 64 output tiles, the
+// panel's columns staged 16 at a time (k-major, one column of padding so the
+// transposing stores fall in distinct banks); each thread owns rows
+// tr + 16 p and columns tc + 16 q, so the tile reads and writes are 128-byte
+// runs, and sums its products from zero: the small products' sum, subtracted
+// once, loses less.  Multiply-adds on registers: on the FP64 tensor cores
+// (mma.sync m8n8k4, whole panels staged) one update of 2,366, 4,766 and 13,184
+// rows takes 40, 137 and 849 us, here 33, 104 and 707 (15.8 TFLOP/s; a factor of
+// 13,248 cells 68.5 -> 58.4 ms).  The width bs (64) stays an argument: with the
+// loop's count known, ptxas schedules it into 41, 112 and 850.
+__global__ void __launch_bounds__(256) k_rf_update(double* A, const double* diag, int n, int k0, int bs)
 {
     if (blockIdx.x == 0)
         for (int e = threadIdx.x; e < RF_B * RF_B; e += 256)
@@ -198,55 +198,36 @@ __global__ void __launch_bounds__(256, 3) k_rf_update(double* A, const double* d
     while (r * (r + 1) / 2 > (int)blockIdx.x) r--;
     const int c = blockIdx.x - r * (r + 1) / 2;
     const int r0 = k0 + RF_B + r * RF_B, c0 = k0 + RF_B + c * RF_B;
-    extern __shared__ double sm[];
-    double* As = sm;
-    double* Bs = (r == c) ? sm : sm + RF_B * RF_LD;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int wr = (warp >> 1) * 16, wc = (warp & 1) * 32, g = lane >> 2, q = lane & 3;
-    // the outputs' present values, on their way while the operands are staged:
-    // accumulator rows g, columns 2 q and 2 q + 1 of each 8 x 8 product.  (Not
-    // what the products are added to: the small products' sum, subtracted once,
-    // loses less.)
-    double old[2][4][2], acc[2][4][2];
+    __shared__ double As[16][RF_B + 1], Bs[16][RF_B + 1];
+    const int tr = threadIdx.x / 16, tc = threadIdx.x % 16;
+    double acc[4][4];
+    for (int p = 0; p < 4; p++)
+        for (int q = 0; q < 4; q++) acc[p][q] = 0.0;
+    for (int kc = 0; kc < bs; kc += 16) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < 16 * RF_B; e += 256) {
+            const int k = e % 16, x = e / 16;
+            const bool in = kc + k < bs;
+            As[k][x] = (in && r0 + x < n) ? A[(size_t)(r0 + x) * n + k0 + kc + k] : 0.0;
+            Bs[k][x] = (in && c0 + x < n) ? A[(size_t)(c0 + x) * n + k0 + kc + k] : 0.0;
+        }
+        __syncthreads();
 #pragma unroll
-    for (int m = 0; m < 2; m++)
+        for (int k = 0; k < 16; k++) {
+            double a[4], b[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++)
+            for (int p = 0; p < 4; p++) { a[p] = As[k][tr + 16 * p]; b[p] = Bs[k][tc + 16 * p]; }
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int i = r0 + wr + 8 * m + g, j = c0 + wc + 8 * u + 2 * q + h;
-                old[m][u][h] = (i < n && j <= i) ? A[(size_t)i * n + j] : 0.0;
-                acc[m][u][h] = 0.0;
-            }
-    for (int e = t; e < RF_B * RF_B; e += 256) {
-        const int row = e / RF_B, k = e % RF_B;
-        As[row * RF_LD + k] = (r0 + row < n) ? A[(size_t)(r0 + row) * n + k0 + k] : 0.0;
-        if (r != c) Bs[row * RF_LD + k] = (c0 + row < n) ? A[(size_t)(c0 + row) * n + k0 + k] : 0.0;
+            for (int p = 0; p < 4; p++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) acc[p][q] = fma(a[p], b[q], acc[p][q]);
+        }
     }
-    __syncthreads();
-#pragma unroll 4
-    for (int k = 0; k < RF_B; k += 4) {
-        double a[2], b[4];
-#pragma unroll
-        for (int m = 0; m < 2; m++) a[m] = As[(wr + 8 * m + g) * RF_LD + k + q];
-#pragma unroll
-        for (int u = 0; u < 4; u++) b[u] = Bs[(wc + 8 * u + g) * RF_LD + k + q];
-#pragma unroll
-        for (int m = 0; m < 2; m++)
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                    : "+d"(acc[m][u][0]), "+d"(acc[m][u][1]) : "d"(a[m]), "d"(b[u]));
-    }
-#pragma unroll
-    for (int m = 0; m < 2; m++)
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int i = r0 + wr + 8 * m + g, j = c0 + wc + 8 * u + 2 * q + h;
-                if (i < n && j <= i) A[(size_t)i * n + j] = old[m][u][h] - acc[m][u][h];
-            }
+    for (int p = 0; p < 4; p++)
+        for (int q = 0; q < 4; q++) {
+            const int i = r0 + tr + 16 * p, j = c0 + tc + 16 * q;
+            if (i < n && j <= i) A[(size_t)i * n + j] = A[(size_t)i * n + j] - acc[p][q];
+        }
 }
 
 // E = L zeta over the lower triangle, one warp per row
@@ -335,16 +316,11 @@ extern "C" int sphk_rf_factor(const int* ip, const double* dp, double* d_C, cuda
     const int T = a.total;
     k_rf_corr<<<dim3((T + 255) / 256, T), 256, 0, st>>>(a, d_C);
     double* d_diag = d_C + (size_t)T * T;
-    const int smem = 2 * RF_B * RF_LD * (int)sizeof(double);
-    if (cudaFuncSetAttribute(k_rf_update, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-        cudaGetLastError();
-        return 1;
-    }
     for (int k0 = 0; k0 < T; k0 += RF_B) {
         const int rest = T - k0 - RF_B;
         const int tiles = (rest > 0) ? (rest + RF_B - 1) / RF_B : 0;
         k_rf_panel<<<tiles > 0 ? tiles : 1, 4 * RF_B, 0, st>>>(d_C, d_diag, T, k0);
-        if (tiles > 0) k_rf_update<<<tiles * (tiles + 1) / 2, 256, smem, st>>>(d_C, d_diag, T, k0);
+        if (tiles > 0) k_rf_update<<<tiles * (tiles + 1) / 2, 256, 0, st>>>(d_C, d_diag, T, k0, RF_B);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
