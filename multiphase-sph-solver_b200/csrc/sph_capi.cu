@@ -690,12 +690,12 @@ void release_field_scratch(sphgpu_ctx* c)
         }
 }
 
-// whether the strain pass takes the artificial-viscosity sums in the steps to
-// come: past inip no step damps again (its own loop also forms the damping and
+// whether the strain pass takes the artificial-viscosity sums from step l on:
+// past inip no step damps again (its own loop also forms the damping and
 // vibration sums)
-void set_visc(sphgpu_ctx* c)
+void set_visc(sphgpu_ctx* c, long long l)
 {
-    const int want = c->precision == SPHGPU_PREC_FP64 && c->P.flv == 0 && c->l_host > c->P.inip;
+    const int want = c->precision == SPHGPU_PREC_FP64 && c->P.flv == 0 && l > c->P.inip;
     if (c->d[0].p.visc == want) return;
     for (int p = 0; p < 2; p++) c->d[p].p.visc = want;
     invalidate_graphs(c);
@@ -1639,7 +1639,7 @@ int run_parts(sphgpu_ctx* c, int upto)
     if (parts & 2) { c->list_split = d->p.split; c->list_bulk = d->p.bulk; }
     if (upto >= 3) {
         if (!c->regu && c->l_host % c->P.step_regu == 0) { c->regu = true; invalidate_graphs(c); }
-        set_visc(c);
+        set_visc(c, c->l_host);
         enqueue_physics(c, d, nullptr);
     }
     CK(cudaGetLastError());
@@ -1795,18 +1795,45 @@ int sphgpu_step(sphgpu_ctx* c, int nsteps)
             if (l % c->P.step_regu == 0) { c->regu = true; invalidate_graphs(c); break; }
     cudaSetDevice(c->device);
     release_field_scratch(c);
-    set_visc(c);
+    const int l0 = c->l_host;
+    set_visc(c, l0);
     if (!c->exec[0] || !c->exec[1]) {
         r = build_graphs(c);
         if (r) return r;
     }
-    const int l0 = c->l_host;
+    // a call whose steps cross inip: the damped ones first, with the graphs of
+    // now, then the others with graphs of their own
+    struct Damped {
+        cudaStream_t st;
+        cudaGraphExec_t exec[2] = {nullptr, nullptr};
+        int steps = 0;
+        long launches = 0;
+        ~Damped()
+        {
+            if (steps > 0) cudaStreamSynchronize(st);      // (a call that failed may have launched some)
+            for (cudaGraphExec_t g : exec)
+                if (g) cudaGraphExecDestroy(g);
+        }
+    } damped{c->st};
+    const long long past = (long long)c->P.inip + 1;
+    if (l0 < past && past < (long long)l0 + nsteps) {
+        std::swap(damped.exec, c->exec);
+        set_visc(c, past);
+        if (c->d[0].p.visc) {
+            damped.steps = (int)(past - l0);
+            damped.launches = c->launches_per_step;
+            r = build_graphs(c);
+            if (r) return r;
+        } else {
+            std::swap(damped.exec, c->exec);
+        }
+    }
     CK(cudaEventRecord(c->ev0, c->st));
     for (int s = 0; s < nsteps; s++) {
         const int p = (c->parity + s) & 1;
         r = sort_if_due(c, p);
         if (r) return r;
-        CK(cudaGraphLaunch(c->exec[p], c->st));
+        CK(cudaGraphLaunch(s < damped.steps ? damped.exec[p] : c->exec[p], c->st));
         c->since_sort++;
     }
     CK(cudaEventRecord(c->ev1, c->st));
@@ -1814,7 +1841,7 @@ int sphgpu_step(sphgpu_ctx* c, int nsteps)
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     c->last_ms = ms;
-    c->last_launches = c->launches_per_step * nsteps;
+    c->last_launches = damped.launches * damped.steps + c->launches_per_step * (nsteps - damped.steps);
     int err = 0, l = 0;
     CK(cudaMemcpy(&err, c->d[0].s.err, sizeof(int), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(&l, c->d[0].s.step, sizeof(int), cudaMemcpyDeviceToHost));
@@ -2487,7 +2514,7 @@ int sphgpu_step_profiled(sphgpu_ctx* c, int nsteps, double* stage_ms)
     int err = 0;
     c->reorder_ms = 0.0;
     for (int s = 0; s < nsteps && err == 0; s++) {
-        set_visc(c);
+        set_visc(c, c->l_host);
         const Dev* d = &c->d[c->parity];
         if (c->reorder_every > 0 && c->since_sort >= c->reorder_every) {
             CK(cudaEventRecord(c->ev0, c->st));
@@ -2583,7 +2610,7 @@ int sphgpu_get_launch(const sphgpu_ctx* c, int* tb, int n)
 int sphgpu_autotune(sphgpu_ctx* c, int steps, const char* cache_path, double* table)
 {
     if (!c || steps <= 0) return SPHGPU_E_ARG;
-    set_visc(c);
+    set_visc(c, c->l_host);
     const std::string key = tune_key(c);
     if (cache_path) {
         if (FILE* f = std::fopen(cache_path, "r")) {
