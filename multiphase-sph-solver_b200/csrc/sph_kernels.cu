@@ -89,7 +89,7 @@ namespace SPH_NS {
 #define SPH_MINB_PAIRW SPH_MINB
 #endif
 // the same trade for the strain pass (6 blocks: 80 registers, a few spills),
-// the density pass (6: 72, none; 7 no faster) and XSPH (8: 64); the
+// the density pass (6: 75, none; 7 no faster) and XSPH (8: 64); the
 // stress-divergence pass ran slower at 5 blocks (2.2 -> 2.5 ms) and keeps 4
 #ifndef SPH_MINB_STRAIN
 #define SPH_MINB_STRAIN 6
