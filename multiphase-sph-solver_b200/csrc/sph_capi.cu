@@ -1538,7 +1538,7 @@ int sphgpu_download_particles(sphgpu_ctx* c, void* particles, int n, size_t stri
             std::memcpy(rec, x, 24);
         }
     };
-    const int smem = 32 * (int)((P / 8) | 1) * 8;      // 29 KB, under the 48 KB of any launch
+    const int smem = 32 * (int)((P / 8) | 1) * 8;      // 19 KB, under the 48 KB of any launch
     // Each host thread takes a share of the particles through its own part of
     // the staging and its own stream: it packs and copies its next piece while
     // it writes the last one into the caller's records, so the copy engine, the
